@@ -71,14 +71,18 @@ constexpr float kLazyMax = 8.0f;          // raise the running maximum only beyo
 #ifndef FBB_EMU_MASK
 #define FBB_EMU_MASK 0x00u
 #endif
+#ifndef FBB_EARLY
+#define FBB_EARLY 4
+#endif
+constexpr int kEarly = FBB_EARLY;
 constexpr unsigned kEmuMask = FBB_EMU_MASK;  // e.g. 0x88: pairs 3 and 7 of 8 (25 %); 0: all on the transcendental unit
 // Register split of the 640-thread (NQ = 2) kernel. It is launched with 96 registers per thread (the most 20 warps can
 // get); setmaxnreg.inc WAITS until the CTA's own pool has the registers, so the split must fit in that pool or the
 // kernel never starts its softmax: 128 * kRegsCtl + 512 * kRegsSoftmax <= 640 * 96. 32 / 112 measured 2 % faster than
 // 40 / 104 (197 vs 201 us at N = 6145): a softmax thread holds 64 scores and up to 32 packed probabilities.
 #ifndef FBB_REGS_CTL
-#define FBB_REGS_CTL 32
-#define FBB_REGS_SOFTMAX 112
+#define FBB_REGS_CTL 56
+#define FBB_REGS_SOFTMAX 104
 #endif
 constexpr int kRegsCtl = FBB_REGS_CTL, kRegsSoftmax = FBB_REGS_SOFTMAX;
 static_assert(128 * kRegsCtl + 512 * kRegsSoftmax <= 640 * 96, "setmaxnreg split exceeds the CTA's register pool");
@@ -88,18 +92,19 @@ static_assert(128 * kRegsCtl + 512 * kRegsSoftmax <= 640 * 96, "setmaxnreg split
 constexpr uint32_t kColTileS = 128, kColO = 256, kColTileOP = 64, kColP = 128;
 
 struct FlashSmem {
-    static constexpr int kQOff = 0;                                  // NQ (<= 2) tiles x 16 KB
-    static constexpr int kKOff = 2 * kTileBytes;                     // stages x 16 KB
+    static constexpr int kQOff = 0;                                  // two items x NQ (<= 2) tiles x 16 KB
+    static constexpr int kKOff = 4 * kTileBytes;                     // stages x 16 KB
     static constexpr int kVOff = kKOff + kKVStages * kTileBytes;     // stages x 16 KB
-    static constexpr int kBarOff = kVOff + kKVStages * kTileBytes;
-    // barriers: q_full, q_empty, k_full[S], v_full[S], k_empty[S], v_empty[S], s_full[2], p_ready[2], pv_done[2], s_free[2], t1_go
-    static constexpr int kNumBars = 2 + 4 * kKVStages + 8 + 1;
+    static constexpr int kOOff = kVOff + kKVStages * kTileBytes;     // output rows on their way out: 16 warps x 2 KB
+    static constexpr int kBarOff = kOOff + 2 * kTileBytes;
+    // barriers: q_full[2], q_empty[2], k_full[S], v_full[S], k_empty[S], v_empty[S], s_full[2], p_ready[2], pv_done[2], s_free[2], t1_go
+    static constexpr int kNumBars = 4 + 4 * kKVStages + 8 + 1;
     static constexpr int kTailOff = kBarOff + kNumBars * 8 + 16;    // TailItems (40 bytes)
     static constexpr int kBytes = kTailOff + 48;
-    // No slack for aligning by hand (the array is declared 1024-byte aligned): 160.4 KB keeps the CTA inside the 164 KB
-    // shared-memory configuration, which leaves the rest of the SM's 256 KB to L1 (the softmax warps spill a few registers).
+    // no slack for aligning by hand (the array is declared 1024-byte aligned)
     static constexpr int kDynamic = kBytes;
 };
+static_assert(FlashSmem::kDynamic <= 232448, "more shared memory than a CTA can have");
 
 // Workspace of the split form: per CTA one slot for the group it starts in the middle. A slot holds, for each of the 16
 // softmax warps, 36 values per lane stored [value][lane] (32 accumulator registers of the 16x256b fragment, then the two
@@ -133,11 +138,14 @@ static __device__ __align__(256) unsigned char g_flash_static_ws[kStaticWsBytes]
 #ifdef FBB_FLASH_TRACE
 // Development aid: per-iteration clock stamps of one softmax warp (CTA 0, lane 0 of warps 4 and 8) and of the UMMA
 // issuer, written to a global buffer set through fbb_flash_trace_buffer(). Not compiled into the shipped library.
-__device__ long long* g_flash_trace = nullptr;
+__device__ unsigned* g_flash_trace = nullptr;
 #define FBB_TRACE(slot, j, k)                                                                                         \
     do {                                                                                                              \
-        if (g_flash_trace != nullptr && blockIdx.x == 0 && lane == 0 && (j) < 64)                                      \
-            g_flash_trace[((slot) * 64 + (j)) * 8 + (k)] = clock64();                                                   \
+        if (trace_to != nullptr && (j) < 160) {                                                                          \
+            unsigned c_;                                                                                                \
+            asm volatile("mov.u32 %0, %%clock;" : "=r"(c_)::"memory");                                                  \
+            trace_to[((slot) * 160 + (j)) * 8 + (k)] = c_;                                                               \
+        }                                                                                                             \
     } while (0)
 #else
 #define FBB_TRACE(slot, j, k) do { } while (0)
@@ -313,25 +321,70 @@ __global__ void __launch_bounds__(128, 16) flash64_side_rows_kernel(const SideAr
     grid_dependency_wait();
 }
 
+// ---- softmax pieces. A warp's 16 rows of a key block in the 16x256b fragment: registers 4k, 4k+1 = keys 8k + 2(lane%4), +1 of
+// row A = lane/4; 4k+2, 4k+3 = the same keys of row B = lane/4 + 8.
+template <int K>  // K groups of 8 keys (even)
+__device__ __forceinline__ void max_frag(const uint32_t* v, float& mxA, float& mxB) {
+    // two chains per row: half the latency before the caller's test
+    float a0 = fmaxf(__uint_as_float(v[0]), __uint_as_float(v[1])), a1 = fmaxf(__uint_as_float(v[4]), __uint_as_float(v[5]));
+    float b0 = fmaxf(__uint_as_float(v[2]), __uint_as_float(v[3])), b1 = fmaxf(__uint_as_float(v[6]), __uint_as_float(v[7]));
+#pragma unroll
+    for (int k = 2; k < K; k += 2) {
+        a0 = fmax3(a0, __uint_as_float(v[4 * k]), __uint_as_float(v[4 * k + 1]));
+        b0 = fmax3(b0, __uint_as_float(v[4 * k + 2]), __uint_as_float(v[4 * k + 3]));
+        a1 = fmax3(a1, __uint_as_float(v[4 * k + 4]), __uint_as_float(v[4 * k + 5]));
+        b1 = fmax3(b1, __uint_as_float(v[4 * k + 6]), __uint_as_float(v[4 * k + 7]));
+    }
+    mxA = fmaxf(a0, a1);
+    mxB = fmaxf(b0, b1);
+}
+__device__ __forceinline__ void mask_frag(uint32_t* v, int key0, int n) {  // 64 keys
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {
+        if (key0 + 8 * k >= n) v[4 * k] = v[4 * k + 2] = 0xff800000u;
+        if (key0 + 8 * k + 1 >= n) v[4 * k + 1] = v[4 * k + 3] = 0xff800000u;
+    }
+}
+// p = 2^(s*sl - m) in fp32, this thread's shares of the row sums, and P as fp16 pairs (the 16x128b fragment)
+template <int K>
+__device__ __forceinline__ void exp_frag(const uint32_t* v, float sl, float mA, float mB, float2& accA, float2& accB, uint32_t* pk) {
+    const float2 sl2 = make_float2(sl, sl), nmA = make_float2(-mA, -mA), nmB = make_float2(-mB, -mB);
+#pragma unroll
+    for (int k = 0; k < K; ++k) {
+        const float2 xA = ffma2(make_float2(__uint_as_float(v[4 * k]), __uint_as_float(v[4 * k + 1])), sl2, nmA);
+        const float2 xB = ffma2(make_float2(__uint_as_float(v[4 * k + 2]), __uint_as_float(v[4 * k + 3])), sl2, nmB);
+        float2 pA, pB;
+        if ((kEmuMask >> (k & 15)) & 1) pA = exp2_emulated(xA);  // these key pairs on the FMA pipes instead of the transcendental unit
+        else pA = make_float2(ex2_approx(xA.x), ex2_approx(xA.y));
+        if ((kEmuMask >> (16 + (k & 15))) & 1) pB = exp2_emulated(xB);
+        else pB = make_float2(ex2_approx(xB.x), ex2_approx(xB.y));
+        accA = fadd2(accA, pA);
+        accB = fadd2(accB, pB);
+        pk[2 * k] = pack_h2(pA.x, pA.y);
+        pk[2 * k + 1] = pack_h2(pB.x, pB.y);
+    }
+}
+
 template <int NQ>
 __global__ void __launch_bounds__(128 + 256 * NQ, 1)
 flash64_umma_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ CUtensorMap tmap_k,
-                    const __grid_constant__ CUtensorMap tmap_v, const FlashArgs a) {
+                    const __grid_constant__ CUtensorMap tmap_v, const __grid_constant__ CUtensorMap tmap_o, const FlashArgs a) {
     using S = FlashSmem;
     extern __shared__ __align__(1024) uint8_t smem_raw[];
     const uint32_t base = smem_u32(smem_raw);
     uint8_t* gen = smem_raw;
     const uint32_t bar0 = base + S::kBarOff;
-    const uint32_t q_full = bar0, q_empty = bar0 + 8u;
-    auto k_full = [&](int s) { return bar0 + 8u * (2 + s); };
-    auto v_full = [&](int s) { return bar0 + 8u * (2 + kKVStages + s); };
-    auto k_empty = [&](int s) { return bar0 + 8u * (2 + 2 * kKVStages + s); };
-    auto v_empty = [&](int s) { return bar0 + 8u * (2 + 3 * kKVStages + s); };
-    auto s_full = [&](int t) { return bar0 + 8u * (2 + 4 * kKVStages + t); };
-    auto p_ready = [&](int t) { return bar0 + 8u * (2 + 4 * kKVStages + 2 + t); };
-    auto pv_done = [&](int t) { return bar0 + 8u * (2 + 4 * kKVStages + 4 + t); };
-    auto s_free = [&](int t) { return bar0 + 8u * (2 + 4 * kKVStages + 6 + t); };
-    const uint32_t t1_go = bar0 + 8u * (2 + 4 * kKVStages + 8);  // completes once: tile 0's issuer has seen its group take the first block
+    auto q_full = [&](int i) { return bar0 + 8u * i; };
+    auto q_empty = [&](int i) { return bar0 + 8u * (2 + i); };
+    auto k_full = [&](int s) { return bar0 + 8u * (4 + s); };
+    auto v_full = [&](int s) { return bar0 + 8u * (4 + kKVStages + s); };
+    auto k_empty = [&](int s) { return bar0 + 8u * (4 + 2 * kKVStages + s); };
+    auto v_empty = [&](int s) { return bar0 + 8u * (4 + 3 * kKVStages + s); };
+    auto s_full = [&](int t) { return bar0 + 8u * (4 + 4 * kKVStages + t); };
+    auto p_ready = [&](int t) { return bar0 + 8u * (4 + 4 * kKVStages + 2 + t); };
+    auto pv_done = [&](int t) { return bar0 + 8u * (4 + 4 * kKVStages + 4 + t); };
+    auto s_free = [&](int t) { return bar0 + 8u * (4 + 4 * kKVStages + 6 + t); };
+    const uint32_t t1_go = bar0 + 8u * (4 + 4 * kKVStages + 8);  // completes once: tile 0's issuer has seen its group take the first block
     volatile uint32_t* s_tmem = reinterpret_cast<volatile uint32_t*>(gen + S::kBarOff + S::kNumBars * 8);
     volatile int* s_abort = reinterpret_cast<volatile int*>(gen + S::kBarOff + S::kNumBars * 8 + 4);
     TailItems* s_tail = reinterpret_cast<TailItems*>(gen + S::kTailOff);
@@ -339,10 +392,16 @@ flash64_umma_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
     const int warp = threadIdx.x >> 5;
     const int lane = threadIdx.x & 31;
     const int nkb = a.nkb;
+#ifdef FBB_FLASH_TRACE
+    if (threadIdx.x == 0 && g_flash_trace != nullptr) { unsigned* q_ = g_flash_trace + 20 * 160 * 8 + blockIdx.x * 4; q_[0] = (unsigned)globaltimer_ns(); unsigned c_; asm volatile("mov.u32 %0, %%clock;" : "=r"(c_)); q_[2] = c_; }
+    unsigned* trace_to = (blockIdx.x == 0 && lane == 0) ? g_flash_trace : nullptr;
+#endif
 
     if (threadIdx.x == 0) {
-        mbar_init(q_full, 1);
-        mbar_init(q_empty, NQ);  // one commit per tile issuer, after the item's last Q K^T
+        for (int i = 0; i < 2; ++i) {
+            mbar_init(q_full(i), 1);
+            mbar_init(q_empty(i), NQ);  // one commit per tile issuer, after the item's last Q K^T
+        }
         for (int s = 0; s < kKVStages; ++s) {
             mbar_init(k_full(s), 1);
             mbar_init(v_full(s), 1);
@@ -378,6 +437,7 @@ flash64_umma_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
         tma_prefetch_desc(&tmap_q);
         tma_prefetch_desc(&tmap_k);
         tma_prefetch_desc(&tmap_v);
+        tma_prefetch_desc(&tmap_o);
     }
     if (warp == 1) {
         __syncwarp();
@@ -414,19 +474,29 @@ flash64_umma_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
         if (lane == 0) {
             int s = 0;
             uint32_t ph = 0;
-            bool ok = true;
-#pragma unroll 1
-            for (int it = 0; it < n_items && ok; ++it) {
+            // Q of an item goes to one of two buffers, so that the next item's is there when a tile gets to it: the tiles run
+            // about a unit and a half apart, and neither waits for the other at the end of an item.
+            auto load_q = [&](int it) -> bool {
                 int w, kb0, kb1;
                 item_at(it, w, kb0, kb1);
                 const int bh = w / a.groups_per_head;
                 const int q0 = (w - bh * a.groups_per_head) * (FQ * NQ);
                 const int b = bh / a.H, h = bh - b * a.H;
-                // Q is single-buffered: the previous item's last Q K^T must have read it (that product is issued one unit
-                // early, so the reload overlaps the previous item's last softmax and write-out)
-                if (!mbar_wait(q_empty, ((uint32_t)it & 1u) ^ 1u, s_abort, DEV_TIMEOUT_SMEM_EMPTY, 32)) { ok = false; break; }
-                mbar_arrive_expect_tx(q_full, NQ * kTileBytes);
-                for (int t = 0; t < NQ; ++t) tma_load_4d(base + S::kQOff + t * kTileBytes, &tmap_q, q_full, 0, h, q0 + t * FQ, b);
+                const int i = it & 1;
+                if (!mbar_wait(q_empty(i), (((uint32_t)it >> 1) & 1u) ^ 1u, s_abort, DEV_TIMEOUT_SMEM_EMPTY, 32)) return false;
+                mbar_arrive_expect_tx(q_full(i), NQ * kTileBytes);
+                for (int t = 0; t < NQ; ++t) tma_load_4d(base + S::kQOff + (2 * i + t) * kTileBytes, &tmap_q, q_full(i), 0, h, q0 + t * FQ, b);
+                return true;
+            };
+            bool ok = n_items == 0 || load_q(0);
+#pragma unroll 1
+            for (int it = 0; it < n_items && ok; ++it) {
+                int w, kb0, kb1;
+                item_at(it, w, kb0, kb1);
+                const int bh = w / a.groups_per_head;
+                const int b = bh / a.H, h = bh - b * a.H;
+                // not before this item's first units: the other buffer is free once both tiles have left the previous item
+                const int kq = it + 1 < n_items ? min(kb0 + kKVStages, kb1 - 1) : -1;
 #pragma unroll 1
                 for (int kb = kb0; kb < kb1; ++kb) {
                     if (!mbar_wait(k_empty(s), ph ^ 1u, s_abort, DEV_TIMEOUT_SMEM_EMPTY, s)) { ok = false; break; }
@@ -436,6 +506,7 @@ flash64_umma_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
                     mbar_arrive_expect_tx(v_full(s), kTileBytes);
                     tma_load_4d(base + S::kVOff + s * kTileBytes, &tmap_v, v_full(s), 0, h, kb * FK, b);
                     if (++s == kKVStages) { s = 0; ph ^= 1u; }
+                    if (kb == kq && !load_q(it + 1)) { ok = false; break; }
                 }
             }
             if (!ok) __nanosleep(20000);
@@ -458,8 +529,8 @@ flash64_umma_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
         const uint32_t dS = tmem_base + t * kColTileS, dO = tmem_base + kColO + t * kColTileOP, aP = dO + kColP;
         auto all_ok = [&](bool mine) { return __all_sync(0xffffffffu, mine) != 0; };
         // S_t = Q_t K^T for one unit: Q buffer of item `it`, K in stage s; `last` = the item's last unit
-        auto issue_qk = [&](int s, bool last) {
-            const uint64_t qd = qd0;
+        auto issue_qk = [&](int it, int s, bool last) {
+            const uint64_t qd = qd0 + (uint64_t)((it & 1) * (2 * kTileBytes >> 4));
             const uint64_t kd = kd0 + (uint64_t)(s * (kTileBytes >> 4));
             umma_ss_warp(dS, qd, kd, idesc_qk, 0u);
             umma_ss_warp(dS, qd + 2u, kd + 2u, idesc_qk, 1u);
@@ -467,7 +538,7 @@ flash64_umma_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
             umma_ss_warp(dS, qd + 6u, kd + 6u, idesc_qk, 1u);
             umma_commit_warp(s_full(t));
             umma_commit_warp(k_empty(s));
-            if (last) umma_commit_warp(q_empty);  // the producer may load the next item's Q
+            if (last) umma_commit_warp(q_empty(it & 1));  // this buffer may be loaded again
         };
         int it = 0, kb = 0, kb1 = 0;
         bool ok = n_items > 0;
@@ -475,7 +546,7 @@ flash64_umma_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
             int w;
             item_at(0, w, kb, kb1);
         }
-        if (ok) ok = all_ok(mbar_wait(q_full, 0, s_abort, DEV_TIMEOUT_TMA_FULL, 100));
+        if (ok) ok = all_ok(mbar_wait(q_full(0), 0, s_abort, DEV_TIMEOUT_TMA_FULL, 100));
         if (ok) ok = all_ok(mbar_wait(k_full(0), 0, s_abort, DEV_TIMEOUT_TMA_FULL, 0));
         // Tile 1 starts once tile 0's group has its first block in registers: the two groups then run slightly out of
         // step, so that one group's load / maximum / store phases overlap the other group's exponentials (measured at
@@ -485,7 +556,7 @@ flash64_umma_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
         if (ok && t == 1 && (n_items > 1 || kb1 - kb > 2)) ok = all_ok(mbar_wait(t1_go, 0, s_abort, DEV_TIMEOUT_TMEM_EMPTY, 50));
         if (ok) {
             tc_fence_after();
-            issue_qk(0, kb + 1 == kb1);
+            issue_qk(0, 0, kb + 1 == kb1);
         }
         int s = 0;
         uint32_t ph = 0, g = 0;
@@ -507,16 +578,16 @@ flash64_umma_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
                 }
             }
             if (have_next) {
+                if (nfirst && !all_ok(mbar_wait(q_full(nit & 1), ((uint32_t)nit >> 1) & 1u, s_abort, DEV_TIMEOUT_TMA_FULL, 101))) { ok = false; break; }
+                if (!all_ok(mbar_wait(k_full(sn), phn, s_abort, DEV_TIMEOUT_TMA_FULL, sn))) { ok = false; break; }
                 if (!all_ok(mbar_wait(s_free(t), g & 1u, s_abort, DEV_TIMEOUT_TMEM_EMPTY, t))) { ok = false; break; }
                 if (NQ == 2 && t == 0 && g == 0 && lane == 0) mbar_arrive(t1_go);  // tile 1 may start (see the gate above)
-                if (nfirst && !all_ok(mbar_wait(q_full, (uint32_t)nit & 1u, s_abort, DEV_TIMEOUT_TMA_FULL, 101))) { ok = false; break; }
-                if (!all_ok(mbar_wait(k_full(sn), phn, s_abort, DEV_TIMEOUT_TMA_FULL, sn))) { ok = false; break; }
                 tc_fence_after();
-                issue_qk(sn, nkb_ + 1 == nkb1);
+                issue_qk(nit, sn, nkb_ + 1 == nkb1);
                 FBB_TRACE(2 + t, g + 1, 3);
             }
-            if (!all_ok(mbar_wait(p_ready(t), g & 1u, s_abort, DEV_TIMEOUT_OTHER, 200 + t))) { ok = false; break; }
             if (!all_ok(mbar_wait(v_full(s), ph, s_abort, DEV_TIMEOUT_TMA_FULL, 16 + s))) { ok = false; break; }
+            if (!all_ok(mbar_wait(p_ready(t), g & 1u, s_abort, DEV_TIMEOUT_OTHER, 200 + t))) { ok = false; break; }
             tc_fence_after();
             FBB_TRACE(2 + t, g, 1);
             const uint64_t vd = vd0 + (uint64_t)(s * (kTileBytes >> 4));
@@ -551,148 +622,21 @@ flash64_umma_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
         const uint32_t tS = tmem_base + ((uint32_t)lane_base << 16) + t * kColTileS;  // this warp's lanes of S_t
         const uint32_t tO = tmem_base + ((uint32_t)lane_base << 16) + kColO + t * kColTileOP;  // ... of O_t; P_t is kColP further
         const float sl = a.scale_log2;
+        const float lazy = kLazyMax / sl;
+        float tA = 0.f, tB = 0.f;  // raw scores beyond which the running maxima are raised
         float mA = -INFINITY, mB = -INFINITY, lA = 0.f, lB = 0.f;  // running maximum and (this thread's share of the) sum
         bool ok = true;
         uint32_t g = 0;  // units done: the phase of the per-tile barriers
 
-#pragma unroll 1
-        for (int it = 0; ok && it < n_items; ++it) {
-            int n;               // key blocks of this item still to do
-            bool to_end;         // the item runs to the group's last key block
-            bool warp_has_rows;  // a warp whose 16 rows all lie beyond N (padding of the last tile) only keeps the barriers moving
-            {
-                int w, kb0, kb1;
-                item_at(it, w, kb0, kb1);
-                n = kb1 - kb0;
-                to_end = kb1 == nkb;
-                warp_has_rows = (w % a.groups_per_head) * (FQ * NQ) + t * FQ + lane_base < a.Nq;
-            }
-            lA = lB = 0.f;
-            bool first = true;
-#pragma unroll 1
-            for (; n > 0; --n, ++g, first = false) {
-                if (u == 0) FBB_TRACE(t, g, 0);
-                if (!mbar_wait(s_full(t), g & 1u, s_abort, DEV_TIMEOUT_TMEM_FULL, t)) { ok = false; break; }
-                tc_fence_after();
-                if (u == 0) FBB_TRACE(t, g, 1);
-                if (!warp_has_rows) {
-                    // This warp only keeps the barriers moving. Its arrival for unit g must wait until the issuer has taken
-                    // p_ready of unit g-1 (it commits pv_done right after issuing that unit's P.V): a tile whose warps are
-                    // all padding would otherwise complete p_ready for g-1 and for g back to back, and the issuer, which
-                    // waits by phase parity, would see the barrier back at the parity it started from and never wake up.
-                    // (Working warps are held the same way by their own wait for pv_done before they overwrite P.)
-                    // S_t is released at once (the next Q K^T needs no more from this warp; its arrival for unit g + 1 can
-                    // only follow S_t(g+1), which the issuer computes after it has seen this unit's release).
-                    tc_fence_before();
-                    __syncwarp();
-                    if (lane == 0) mbar_arrive(s_free(t));
-                    if (g > 0 && !mbar_wait(pv_done(t), (g - 1u) & 1u, s_abort, DEV_TIMEOUT_OTHER, 210 + t)) { ok = false; break; }
-                    if (lane == 0) mbar_arrive(p_ready(t));
-                    continue;
-                }
-                uint32_t r[64];
-                tmem_ld_16x256b_x16(tS, r);
-                tmem_wait_ld();
-                tc_fence_before();
-                __syncwarp();
-                if (lane == 0) mbar_arrive(s_free(t));  // S_t is in registers: the next Q K^T may overwrite it
-                float va[64];
-#pragma unroll
-                for (int i = 0; i < 64; ++i) va[i] = __uint_as_float(r[i]);
-                if (to_end && n == 1 && (a.N & (FK - 1)) != 0) {  // the group's last key block is ragged: mask keys >= N
-                    const int key0 = (nkb - 1) * FK + 2 * cq;
-#pragma unroll
-                    for (int k = 0; k < 16; ++k) {
-                        if (key0 + 8 * k >= a.N) va[4 * k] = va[4 * k + 2] = -INFINITY;
-                        if (key0 + 8 * k + 1 >= a.N) va[4 * k + 1] = va[4 * k + 3] = -INFINITY;
-                    }
-                }
-                float mxA = fmaxf(va[0], va[1]), mxB = fmaxf(va[2], va[3]);
-#pragma unroll
-                for (int k = 1; k < 16; ++k) {
-                    mxA = fmax3(mxA, va[4 * k], va[4 * k + 1]);
-                    mxB = fmax3(mxB, va[4 * k + 2], va[4 * k + 3]);
-                }
-                mxA = fmaxf(mxA, __shfl_xor_sync(0xffffffffu, mxA, 1));
-                mxB = fmaxf(mxB, __shfl_xor_sync(0xffffffffu, mxB, 1));
-                mxA = fmaxf(mxA, __shfl_xor_sync(0xffffffffu, mxA, 2)) * sl;
-                mxB = fmaxf(mxB, __shfl_xor_sync(0xffffffffu, mxB, 2)) * sl;
-                if (u == 0) FBB_TRACE(t, g, 2);
-                // ---- running maxima: raised only when this block exceeds them by more than 2^kLazyMax
-                if (first) {
-                    mA = mxA;
-                    mB = mxB;
-                } else if (__any_sync(0xffffffffu, mxA > mA + kLazyMax || mxB > mB + kLazyMax)) {
-                    // O_t is still being accumulated by the previous unit's P.V
-                    if (!mbar_wait(pv_done(t), (g - 1u) & 1u, s_abort, DEV_TIMEOUT_TMEM_FULL, 8 + t)) { ok = false; break; }
-                    tc_fence_after();
-                    const float nA = fmaxf(mA, mxA), nB = fmaxf(mB, mxB);
-                    const float cA = ex2_approx(mA - nA), cB = ex2_approx(mB - nB);
-                    // in place, 16 columns at a time: this path is rare, and a whole O tile in registers on top of the
-                    // 64 scores held here would make the compiler spill in the hot loop around it
-#pragma unroll 1
-                    for (int c = 0; c < 4; ++c) {
-                        uint32_t o[8];
-                        tmem_ld_16x256b_x2(tO + 16u * c, o);
-                        tmem_wait_ld();
-#pragma unroll
-                        for (int k = 0; k < 2; ++k) {
-                            o[4 * k] = __float_as_uint(__uint_as_float(o[4 * k]) * cA);
-                            o[4 * k + 1] = __float_as_uint(__uint_as_float(o[4 * k + 1]) * cA);
-                            o[4 * k + 2] = __float_as_uint(__uint_as_float(o[4 * k + 2]) * cB);
-                            o[4 * k + 3] = __float_as_uint(__uint_as_float(o[4 * k + 3]) * cB);
-                        }
-                        tmem_st_16x256b_x2(tO + 16u * c, o);
-                    }
-                    lA *= cA;
-                    lB *= cB;
-                    mA = nA;
-                    mB = nB;
-                }
-                // ---- p = 2^(s*sl - m) in fp32; row sums in fp32; P as fp16 pairs back to tensor memory
-                const float2 sl2 = make_float2(sl, sl), nmA = make_float2(-mA, -mA), nmB = make_float2(-mB, -mB);
-                float2 accA = make_float2(0.f, 0.f), accB = make_float2(0.f, 0.f);
-                uint32_t pk[32];
-#pragma unroll
-                for (int k = 0; k < 16; ++k) {
-                    const float2 xA = ffma2(make_float2(va[4 * k], va[4 * k + 1]), sl2, nmA);
-                    const float2 xB = ffma2(make_float2(va[4 * k + 2], va[4 * k + 3]), sl2, nmB);
-                    float2 pA, pB;
-                    if ((kEmuMask >> (k & 7)) & 1) {  // this key pair on the FMA pipes instead of the transcendental unit
-                        pA = exp2_emulated(xA);
-                        pB = exp2_emulated(xB);
-                    } else {
-                        pA = make_float2(ex2_approx(xA.x), ex2_approx(xA.y));
-                        pB = make_float2(ex2_approx(xB.x), ex2_approx(xB.y));
-                    }
-                    accA = fadd2(accA, pA);
-                    accB = fadd2(accB, pB);
-                    pk[2 * k] = pack_h2(pA.x, pA.y);
-                    pk[2 * k + 1] = pack_h2(pB.x, pB.y);
-                }
-                // P_t is read by the previous unit's P.V until that product has completed: waiting here, not before the
-                // exponentials, keeps the issue and run time of that product (~900 clocks) off the softmax warps' path
-                if (g > 0) {
-                    if (!mbar_wait(pv_done(t), (g - 1u) & 1u, s_abort, DEV_TIMEOUT_TMEM_FULL, 8 + t)) { ok = false; break; }
-                    tc_fence_after();
-                }
-                tmem_st_16x128b_x16(tO + kColP, pk);
-                if (u == 0) FBB_TRACE(t, g, 3);
-                tmem_wait_st();
-                tc_fence_before();
-                __syncwarp();
-                if (lane == 0) mbar_arrive(p_ready(t));
-                if (u == 0) FBB_TRACE(t, g, 4);
-                lA += accA.x + accA.y;
-                lB += accB.x + accB.y;
-            }
-            if (!ok || !warp_has_rows) continue;
-
-            // ---- end of an item: wait for its last P.V, then write the rows, or hand over / merge a split group
-            if (!mbar_wait(pv_done(t), (g - 1u) & 1u, s_abort, DEV_TIMEOUT_TMEM_FULL, 8 + t)) { ok = false; break; }
-            tc_fence_after();
+        // An item's rows are written (or handed over, or merged) when its last P.V has completed, which is only waited for in
+        // the next item's first unit, after that unit's exponentials: `done` is the item, lA .. mB its sums and maxima.
+        int done = -1;
+        float dlA = 0.f, dlB = 0.f, dmA = 0.f, dmB = 0.f;
+        auto finish = [&]() -> bool {
             int w, kb0, kb1;
-            item_at(it, w, kb0, kb1);
+            item_at(done, w, kb0, kb1);
+            done = -1;
+            float lA = dlA, lB = dlB, mA = dmA, mB = dmB;
             uint32_t o[32];
             tmem_ld_16x256b_x8(tO, o);
             tmem_wait_ld();
@@ -709,12 +653,12 @@ flash64_umma_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
                 __threadfence();
                 __syncwarp();
                 if (lane == 0) st_release_gpu(a.ws_flags + (size_t)blockIdx.x * kSlotWarps + wslot, 1u);
-                continue;
+                return true;
             }
             if (kb1 != nkb) {
                 // The next CTA holds the rest of this group's keys (the first thing it did in its tail share).
                 unsigned* flag = a.ws_flags + (size_t)(blockIdx.x + 1u) * kSlotWarps + wslot;
-                if (!wait_slot_flag(flag, lane, s_abort, 300 + wslot)) { ok = false; break; }
+                if (!wait_slot_flag(flag, lane, s_abort, 300 + wslot)) return false;
                 const float* src = a.ws_data + ((size_t)(blockIdx.x + 1u) * kSlotWarps + wslot) * (kSlotValues * 32) + lane;
                 const float pmA = __ldcg(src + 32 * 32), pmB = __ldcg(src + 33 * 32);
                 const float nA = fmaxf(mA, pmA), nB = fmaxf(mB, pmB);
@@ -740,21 +684,250 @@ flash64_umma_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
             const float invA = 1.f / lA, invB = 1.f / lB;
             const int bh = w / a.groups_per_head;
             const int b = bh / a.H, h = bh - b * a.H;
-            const int rowA = (w - bh * a.groups_per_head) * (FQ * NQ) + t * FQ + lane_base + (lane >> 2);  // this thread's rows: rowA, rowA + 8
-            __half* dstA = a.o + (int64_t)b * a.o_sb + (int64_t)rowA * a.o_sn + (int64_t)h * a.o_sh + 2 * cq;
-            __half* dstB = dstA + 8 * a.o_sn;
+            // The warp's 16 rows of 128 bytes leave through its own 2 KB of shared memory and one TMA store, which clips rows
+            // at Nq: the fragment is four stmatrix of 8x8 tiles (lane i supplies the address of row i%8 of tile i/8), 16-byte
+            // units swizzled as the tensor map's 128-byte mode expects them.
+            if (lane == 0) bulk_wait_read_all();  // the previous item's rows have left
+            __syncwarp();
+            const uint32_t st = base + S::kOOff + (uint32_t)(t * 8 + u) * 2048u;
+            const uint32_t strow = (uint32_t)(lane & 15);              // tiles 0, 1 of a call: rows 0-7, 8-15 of one column group; 2, 3: the next one
 #pragma unroll
-            for (int k = 0; k < 8; ++k) {
-                if (rowA < a.Nq)
-                    *reinterpret_cast<uint32_t*>(dstA + 8 * k) = pack_h2(__uint_as_float(o[4 * k]) * invA, __uint_as_float(o[4 * k + 1]) * invA);
-                if (rowA + 8 < a.Nq)
-                    *reinterpret_cast<uint32_t*>(dstB + 8 * k) = pack_h2(__uint_as_float(o[4 * k + 2]) * invB, __uint_as_float(o[4 * k + 3]) * invB);
+            for (int k = 0; k < 8; k += 2) {
+                const uint32_t unit = (uint32_t)(k + (lane >> 4)) ^ (strow & 7u);
+                stmatrix_x4(st + strow * 128u + unit * 16u,
+                            pack_h2(__uint_as_float(o[4 * k]) * invA, __uint_as_float(o[4 * k + 1]) * invA),
+                            pack_h2(__uint_as_float(o[4 * k + 2]) * invB, __uint_as_float(o[4 * k + 3]) * invB),
+                            pack_h2(__uint_as_float(o[4 * k + 4]) * invA, __uint_as_float(o[4 * k + 5]) * invA),
+                            pack_h2(__uint_as_float(o[4 * k + 6]) * invB, __uint_as_float(o[4 * k + 7]) * invB));
             }
+            fence_proxy_async_smem();
+            __syncwarp();
+            if (lane == 0) {
+                tma_store_4d(&tmap_o, st, 0, h, (w - bh * a.groups_per_head) * (FQ * NQ) + t * FQ + lane_base, b);
+                bulk_commit();
+            }
+            return true;
+        };
+
+#pragma unroll 1
+        for (int it = 0; ok && it < n_items; ++it) {
+            int n;               // key blocks of this item still to do
+            bool to_end;         // the item runs to the group's last key block
+            bool warp_has_rows;  // a warp whose 16 rows all lie beyond N (padding of the last tile) only keeps the barriers moving
+            {
+                int w, kb0, kb1;
+                item_at(it, w, kb0, kb1);
+                n = kb1 - kb0;
+                to_end = kb1 == nkb;
+                warp_has_rows = (w % a.groups_per_head) * (FQ * NQ) + t * FQ + lane_base < a.Nq;
+            }
+            if (!warp_has_rows) {
+#pragma unroll 1
+                for (; n > 0; --n, ++g) {
+                    // This warp only keeps the barriers moving. Its arrival for unit g must wait until the issuer has taken
+                    // p_ready of unit g-1 (it commits pv_done right after issuing that unit's P.V): a tile whose warps are
+                    // all padding would otherwise complete p_ready for g-1 and for g back to back, and the issuer, which
+                    // waits by phase parity, would see the barrier back at the parity it started from and never wake up.
+                    // (Working warps are held the same way by their own wait for pv_done before they overwrite P.)
+                    // S_t is released at once (the next Q K^T needs no more from this warp; its arrival for unit g + 1 can
+                    // only follow S_t(g+1), which the issuer computes after it has seen this unit's release).
+                    if (!mbar_wait(s_full(t), g & 1u, s_abort, DEV_TIMEOUT_TMEM_FULL, t)) { ok = false; break; }
+                    tc_fence_after();
+                    tc_fence_before();
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(s_free(t));
+                    if (g > 0 && !mbar_wait(pv_done(t), (g - 1u) & 1u, s_abort, DEV_TIMEOUT_OTHER, 210 + t)) { ok = false; break; }
+                    tc_fence_after();
+                    if (done >= 0 && !finish()) { ok = false; break; }
+                    if (lane == 0) mbar_arrive(p_ready(t));
+                }
+                continue;
+            }
+            const bool ragged = to_end && (a.N & (FK - 1)) != 0;  // the group's last key block has keys beyond N
+            const int key0 = (nkb - 1) * FK + 2 * cq;
+            {
+                // ---- the item's first unit takes the running maxima
+                if (!mbar_wait(s_full(t), g & 1u, s_abort, DEV_TIMEOUT_TMEM_FULL, t)) { ok = false; break; }
+                tc_fence_after();
+                uint32_t sc[64], pk[32];
+                tmem_ld_16x256b_x16(tS, sc);
+                tmem_wait_ld();
+                tmem_tie32(sc);
+                tmem_tie32(sc + 32);
+                tc_fence_before();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(s_free(t));
+                if (ragged && n == 1) {
+                    mask_frag(sc, key0, a.N);
+                    mask_frag(sc + 32, key0 + 64, a.N);
+                }
+                float mxA, mxB;
+                max_frag<16>(sc, mxA, mxB);
+                mxA = fmaxf(mxA, __shfl_xor_sync(0xffffffffu, mxA, 1));
+                mxB = fmaxf(mxB, __shfl_xor_sync(0xffffffffu, mxB, 1));
+                mxA = fmaxf(mxA, __shfl_xor_sync(0xffffffffu, mxA, 2));
+                mxB = fmaxf(mxB, __shfl_xor_sync(0xffffffffu, mxB, 2));
+                mA = mxA * sl;
+                mB = mxB * sl;
+                tA = mxA + lazy;
+                tB = mxB + lazy;
+                float2 accA = make_float2(0.f, 0.f), accB = make_float2(0.f, 0.f);
+                exp_frag<16>(sc, sl, mA, mB, accA, accB, pk);
+                if (g > 0) {
+                    if (!mbar_wait(pv_done(t), (g - 1u) & 1u, s_abort, DEV_TIMEOUT_TMEM_FULL, 8 + t)) { ok = false; break; }
+                    tc_fence_after();
+                }
+                tmem_st_16x128b_x16(tO + kColP, pk);
+                if (done >= 0 && !finish()) { ok = false; break; }  // before this item's first P.V overwrites O_t
+                tmem_wait_st();
+                tc_fence_before();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(p_ready(t));
+                lA = accA.x + accA.y;
+                lB = accB.x + accB.y;
+                --n;
+                ++g;
+            }
+            int plain = n - (ragged ? 1 : 0);
+#pragma unroll 1
+            while (n > 0) {
+                // ---- the units that are all alike
+                float2 accA = make_float2(0.f, 0.f), accB = make_float2(0.f, 0.f);
+#pragma unroll 1
+                for (; plain > 0; --plain, --n, ++g) {
+                    FBB_TRACE(4 + u + 8 * t, g, 0);
+                    if (!mbar_wait(s_full(t), g & 1u, s_abort, DEV_TIMEOUT_TMEM_FULL, t)) { ok = false; break; }
+                    tc_fence_after();
+                    FBB_TRACE(4 + u + 8 * t, g, 1);
+                    uint32_t sc[64], pk[32];
+                    tmem_ld_16x256b_x16(tS, sc);
+                    tmem_wait_ld();
+                    tmem_tie32(sc);
+                    tmem_tie32(sc + 32);
+                    float mxA, mxB;
+                    max_frag<16>(sc, mxA, mxB);
+                    accA = make_float2(0.f, 0.f);
+                    accB = make_float2(0.f, 0.f);
+                    exp_frag<kEarly>(sc, sl, mA, mB, accA, accB, pk);
+                    if (__any_sync(0xffffffffu, mxA > tA || mxB > tB)) break;
+                    tc_fence_before();
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(s_free(t));  // S_t is in registers: the next Q K^T may overwrite it
+                    FBB_TRACE(4 + u + 8 * t, g, 2);
+                    exp_frag<16 - kEarly>(sc + 4 * kEarly, sl, mA, mB, accA, accB, pk + 2 * kEarly);
+                    // P_t is read by the previous unit's P.V until that product has completed: waiting here, not before the
+                    // exponentials, keeps the issue and run time of that product off the softmax warps' path
+                    if (!mbar_wait(pv_done(t), (g - 1u) & 1u, s_abort, DEV_TIMEOUT_TMEM_FULL, 8 + t)) { ok = false; break; }
+                    tc_fence_after();
+                    tmem_st_16x128b_x16(tO + kColP, pk);
+                    FBB_TRACE(4 + u + 8 * t, g, 3);
+                    tmem_wait_st();
+                    tc_fence_before();
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(p_ready(t));
+                    FBB_TRACE(4 + u + 8 * t, g, 4);
+                    lA += accA.x + accA.y;
+                    lB += accB.x + accB.y;
+                }
+                if (!ok || n == 0) break;
+                // ---- the others, half a key block at a time from tensor memory: a block that exceeds a row's running maximum by
+                // more than 2^kLazyMax (raises them and rescales O and the sums) and the ragged last block (masks keys)
+                const bool mask = plain == 0;
+                if (!mbar_wait(s_full(t), g & 1u, s_abort, DEV_TIMEOUT_TMEM_FULL, t)) { ok = false; break; }
+                tc_fence_after();
+                float mxA = -INFINITY, mxB = -INFINITY;
+#pragma unroll 1
+                for (int h = 0; h < 2; ++h) {
+                    uint32_t v[32];
+                    tmem_ld_16x256b_x8(tS + 64u * h, v);
+                    tmem_wait_ld();
+                    tmem_tie32(v);
+                    if (mask) mask_frag(v, key0 + 64 * h, a.N);
+                    float xA, xB;
+                    max_frag<8>(v, xA, xB);
+                    mxA = fmaxf(mxA, xA);
+                    mxB = fmaxf(mxB, xB);
+                }
+                mxA = fmaxf(mxA, __shfl_xor_sync(0xffffffffu, mxA, 1));
+                mxB = fmaxf(mxB, __shfl_xor_sync(0xffffffffu, mxB, 1));
+                mxA = fmaxf(mxA, __shfl_xor_sync(0xffffffffu, mxA, 2));
+                mxB = fmaxf(mxB, __shfl_xor_sync(0xffffffffu, mxB, 2));
+                // P_t and O_t are in use by the previous unit's P.V until that product has completed
+                if (!mbar_wait(pv_done(t), (g - 1u) & 1u, s_abort, DEV_TIMEOUT_TMEM_FULL, 8 + t)) { ok = false; break; }
+                tc_fence_after();
+                if (__any_sync(0xffffffffu, mxA > tA || mxB > tB)) {
+                    const float nA = fmaxf(mA, mxA * sl), nB = fmaxf(mB, mxB * sl);
+                    const float cA = ex2_approx(mA - nA), cB = ex2_approx(mB - nB);
+#pragma unroll 1
+                    for (int c = 0; c < 4; ++c) {
+                        uint32_t o[8];
+                        tmem_ld_16x256b_x2(tO + 16u * c, o);
+                        tmem_wait_ld();
+#pragma unroll
+                        for (int k = 0; k < 2; ++k) {
+                            o[4 * k] = __float_as_uint(__uint_as_float(o[4 * k]) * cA);
+                            o[4 * k + 1] = __float_as_uint(__uint_as_float(o[4 * k + 1]) * cA);
+                            o[4 * k + 2] = __float_as_uint(__uint_as_float(o[4 * k + 2]) * cB);
+                            o[4 * k + 3] = __float_as_uint(__uint_as_float(o[4 * k + 3]) * cB);
+                        }
+                        tmem_st_16x256b_x2(tO + 16u * c, o);
+                    }
+                    lA *= cA;
+                    lB *= cB;
+                    mA = nA;
+                    mB = nB;
+                    tA = fmaxf(tA, mxA + lazy);
+                    tB = fmaxf(tB, mxB + lazy);
+                }
+                accA = make_float2(0.f, 0.f);
+                accB = make_float2(0.f, 0.f);
+#pragma unroll 1
+                for (int h = 0; h < 2; ++h) {
+                    uint32_t v[32], pk[16];
+                    if (mask && (nkb - 1) * FK + 64 * h >= a.N) {  // no key in this half
+#pragma unroll
+                        for (int i = 0; i < 16; ++i) pk[i] = 0u;
+                    } else {
+                        tmem_ld_16x256b_x8(tS + 64u * h, v);
+                        tmem_wait_ld();
+                        tmem_tie32(v);
+                        if (mask) mask_frag(v, key0 + 64 * h, a.N);
+                        exp_frag<8>(v, sl, mA, mB, accA, accB, pk);
+                    }
+                    tmem_st_16x128b_x8(tO + kColP + 32u * h, pk);
+                }
+                tc_fence_before();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(s_free(t));
+                tmem_wait_st();
+                tc_fence_before();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(p_ready(t));
+                lA += accA.x + accA.y;
+                lB += accB.x + accB.y;
+                --n;
+                --plain;
+                ++g;
+            }
+            if (!ok) continue;
+            done = it;
+            dlA = lA;
+            dlB = lB;
+            dmA = mA;
+            dmB = mB;
         }
+        if (ok && done >= 0 && mbar_wait(pv_done(t), (g - 1u) & 1u, s_abort, DEV_TIMEOUT_TMEM_FULL, 8 + t)) {
+            tc_fence_after();
+            finish();
+        }
+        if (lane == 0) bulk_wait_all();
     }
 
     tc_fence_before();
     __syncthreads();
+#ifdef FBB_FLASH_TRACE
+    if (threadIdx.x == 0 && g_flash_trace != nullptr) { unsigned* q_ = g_flash_trace + 20 * 160 * 8 + blockIdx.x * 4; q_[1] = (unsigned)globaltimer_ns(); unsigned c_; asm volatile("mov.u32 %0, %%clock;" : "=r"(c_)); q_[3] = c_; }
+#endif
     if (warp == 1) {
         __syncwarp();
         tc_fence_after();
@@ -763,7 +936,7 @@ flash64_umma_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
 }
 
 template <int NQ>
-static int launch_flash_variant(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, FlashArgs a, int B, void* ws,
+static int launch_flash_variant(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const CUtensorMap& to, FlashArgs a, int B, void* ws,
                                 int64_t ws_bytes, cudaStream_t stream) {
     static bool configured[64] = {};
     int dev = 0;
@@ -801,14 +974,14 @@ static int launch_flash_variant(const CUtensorMap& tq, const CUtensorMap& tk, co
         a.ws_data = reinterpret_cast<float*>(reinterpret_cast<uint8_t*>(ws) + flag_region_bytes(sms));
     }
     if ((int64_t)a.rounds * a.nkb + 2 * (int64_t)a.nkb * 2 > 0x7FFFFFFFll) return fail(FBB_ERR_SHAPE, "flash64: too many key blocks per CTA");
-    cudaError_t e = launch_pdl(kern, dim3((unsigned)ctas), dim3(128 + 256 * NQ), FlashSmem::kDynamic, stream, tq, tk, tv, a);
+    cudaError_t e = launch_pdl(kern, dim3((unsigned)ctas), dim3(128 + 256 * NQ), FlashSmem::kDynamic, stream, tq, tk, tv, to, a);
     if (e != cudaSuccess) return fail((int)e, "flash64_umma_kernel launch: %s", cudaGetErrorString(e));
     return FBB_OK;
 }
 
 #ifdef FBB_FLASH_TRACE
 extern "C" int fbb_flash_trace_buffer(void* buf) {
-    long long* p = reinterpret_cast<long long*>(buf);
+    unsigned* p = reinterpret_cast<unsigned*>(buf);
     return (int)cudaMemcpyToSymbol(g_flash_trace, &p, sizeof(p));
 }
 #endif
@@ -953,9 +1126,19 @@ int launch_flash64(const void* q, const void* k, const void* v, void* o, int B, 
     if (side > 0 && ws_bytes < flash64_workspace_bytes())
         return fail(FBB_ERR_SHAPE, "flash64: workspace of %lld bytes, %lld needed", (long long)ws_bytes, (long long)flash64_workspace_bytes());
     a.Nq = N - side;
+    CUtensorMap to;  // 16 rows of one head at a time; rows from Nq on are not this kernel's
+    {
+        const uint64_t odims[4] = {64, (uint64_t)H, (uint64_t)a.Nq, (uint64_t)B};
+        const uint32_t obox[4] = {64, 1, 16, 1};
+        int64_t st[4] = {1, os[2], os[1], os[0]};
+        if (H == 1 && st[1] == 0) st[1] = 64;
+        if (B == 1 && st[3] == 0) st[3] = st[2] * (int64_t)N;
+        const int rc = make_tmap_f16(&to, o, 4, odims, st, obox);
+        if (rc != FBB_OK) return rc;
+    }
     int rc;
-    if (two_tiles_per_cta(B, a.Nq, H)) rc = launch_flash_variant<2>(tq, tk, tv, a, B, ws, ws_bytes, stream);
-    else rc = launch_flash_variant<1>(tq, tk, tv, a, B, ws, ws_bytes, stream);  // (never with side rows: see side_rows_for)
+    if (two_tiles_per_cta(B, a.Nq, H)) rc = launch_flash_variant<2>(tq, tk, tv, to, a, B, ws, ws_bytes, stream);
+    else rc = launch_flash_variant<1>(tq, tk, tv, to, a, B, ws, ws_bytes, stream);  // (never with side rows: see side_rows_for)
     if (rc != FBB_OK || side == 0) return rc;
     return launch_side_rows(a, q, k, v, B, qs, ks, vs, side, ws, stream);
 }
