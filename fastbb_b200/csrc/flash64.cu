@@ -25,11 +25,18 @@
 //   warps 4..11/12..19 softmax group t, 16 query rows per warp: tcgen05.ld 16x256b hands thread i the key pairs
 //                   8k + 2(i%4), +1 of rows i/4 and i/4 + 8 (the m16n8 accumulator fragment), so a row's maximum and sum
 //                   take two shuffles among the four threads that share it, and P (fp16 pairs) goes back with the
-//                   matching 16x128b store. The 128-key block is loaded at once and S is released immediately; the
-//                   maximum is taken with 3-input max, p = 2^(s*scale*log2e - m) with packed f32x2 FMAs.
-//                   The running maximum m is only raised when a block exceeds it by more than 2^8 (then O_t and the
-//                   running sum are rescaled in place, a rare event after the first blocks); otherwise P is taken
-//                   relative to the older maximum, which keeps it <= 256 and exactly as accurate in fp16.
+//                   matching 16x128b store. The 128-key block is loaded at once; the maximum is taken with 3-input max,
+//                   p = 2^(s*scale*log2e - m) with packed f32x2 FMAs. The running maximum m is only raised when a block
+//                   exceeds it by more than 2^8 (then O_t and the running sum are rescaled in place, a rare event after
+//                   the first blocks); otherwise P is taken relative to the older maximum, which keeps it <= 256 and
+//                   exactly as accurate in fp16. The loop over an item's blocks holds only what every block needs: each
+//                   thread compares its own share of a row with the row's limit and the warp votes (no shuffles), and a
+//                   block that has to raise the maximum, or is ragged, leaves for a second loop that reads S again from
+//                   tensor memory in halves. An item's first block (which takes the maximum) stands before the loop, its
+//                   rows are written by 16-row TMA stores in the NEXT item's first block, behind that block's
+//                   exponentials, and Q has two buffers, so that neither tile stops between items. With one loop for all
+//                   of this and the write-out between items: 1531 / 213.6 / 81.8 us at N = 16385 / 6145 / 4097 (16 / 16 /
+//                   12 heads, back to back on one B200); now 1303 / 193.0 / 73.5.
 //                   Four softmax warps share each SM sub-partition and cover one another's waits (measured against
 //                   one-thread-per-row groups of four warps: 740 -> 849 TFLOP/s at N = 16385).
 // With NQ = 2 the two groups alternate on the tensor core (S of one tile is computed while the other tile is in its
@@ -65,26 +72,16 @@ constexpr int FK = 128;       // keys per block
 constexpr int kKVStages = 4;
 constexpr int kTileBytes = 128 * 64 * 2;  // one [128 x 64] fp16 tile
 constexpr float kLazyMax = 8.0f;          // raise the running maximum only beyond 2^8
-// Which of every 8 consecutive key pairs get their exponentials from the polynomial on the FMA pipes (bit i = pair i).
-// Measured on B200 (N = 16385, 16 heads): mask 0 -> 849, 0x88 -> 841, 0xAA -> 700 TFLOP/s: the extra FMA / ALU
-// instructions cost what the transcendental unit saves, so the shipped default is 0 (the code path stays for tuning).
-#ifndef FBB_EMU_MASK
-#define FBB_EMU_MASK 0x00u
-#endif
-#ifndef FBB_EARLY
-#define FBB_EARLY 4
-#endif
-constexpr int kEarly = FBB_EARLY;
-constexpr unsigned kEmuMask = FBB_EMU_MASK;  // e.g. 0x88: pairs 3 and 7 of 8 (25 %); 0: all on the transcendental unit
+// Key groups of eight whose exponentials a thread takes before the test of the running maximum is known: the test's vote then
+// costs no wait, and S_t is released that much later. Measured on B200 (us at N = 16385 / 6145 / 1041 tokens, 16 / 16 / 12
+// heads): 0 -> 1315 / 194.0 / 14.4, 2 -> 1332 / 194.3 / 13.9, 4 -> 1303 / 193.0 / 13.5, 8 -> 1324 / 190.4 / 13.7.
+constexpr int kEarly = 4;
 // Register split of the 640-thread (NQ = 2) kernel. It is launched with 96 registers per thread (the most 20 warps can
 // get); setmaxnreg.inc WAITS until the CTA's own pool has the registers, so the split must fit in that pool or the
-// kernel never starts its softmax: 128 * kRegsCtl + 512 * kRegsSoftmax <= 640 * 96. 32 / 112 measured 2 % faster than
-// 40 / 104 (197 vs 201 us at N = 6145): a softmax thread holds 64 scores and up to 32 packed probabilities.
-#ifndef FBB_REGS_CTL
-#define FBB_REGS_CTL 56
-#define FBB_REGS_SOFTMAX 104
-#endif
-constexpr int kRegsCtl = FBB_REGS_CTL, kRegsSoftmax = FBB_REGS_SOFTMAX;
+// kernel never starts its softmax: 128 * kRegsCtl + 512 * kRegsSoftmax <= 640 * 96. A softmax thread holds 64 scores and up to
+// 32 packed probabilities; 104 hold them without spilling, and the issuers keep their loop state in registers with 56
+// (us at N = 16385 / 6145 / 4097, 16 / 16 / 12 heads: 1303 / 193 / 73.5; with 32 / 112: 1358 / 200 / 76.5).
+constexpr int kRegsCtl = 56, kRegsSoftmax = 104;
 static_assert(128 * kRegsCtl + 512 * kRegsSoftmax <= 640 * 96, "setmaxnreg split exceeds the CTA's register pool");
 
 // tensor-memory columns of tile t: S_t (128 columns) at t * kColTileS, O_t (fp32, 64 columns) at kColO + t * kColTileOP,
@@ -353,11 +350,7 @@ __device__ __forceinline__ void exp_frag(const uint32_t* v, float sl, float mA, 
     for (int k = 0; k < K; ++k) {
         const float2 xA = ffma2(make_float2(__uint_as_float(v[4 * k]), __uint_as_float(v[4 * k + 1])), sl2, nmA);
         const float2 xB = ffma2(make_float2(__uint_as_float(v[4 * k + 2]), __uint_as_float(v[4 * k + 3])), sl2, nmB);
-        float2 pA, pB;
-        if ((kEmuMask >> (k & 15)) & 1) pA = exp2_emulated(xA);  // these key pairs on the FMA pipes instead of the transcendental unit
-        else pA = make_float2(ex2_approx(xA.x), ex2_approx(xA.y));
-        if ((kEmuMask >> (16 + (k & 15))) & 1) pB = exp2_emulated(xB);
-        else pB = make_float2(ex2_approx(xB.x), ex2_approx(xB.y));
+        const float2 pA = make_float2(ex2_approx(xA.x), ex2_approx(xA.y)), pB = make_float2(ex2_approx(xB.x), ex2_approx(xB.y));
         accA = fadd2(accA, pA);
         accB = fadd2(accB, pB);
         pk[2 * k] = pack_h2(pA.x, pA.y);
