@@ -51,7 +51,7 @@ static int run_block(const fbb_block_desc& d, const fbb_block_desc* next, bool y
     int rc = FBB_OK;
     if (!y_ready) rc = launch_layernorm(x, y, d.ln1_w, d.ln1_b, T, C, C, C, d.eps1, FBB_DTYPE_F16, FBB_DTYPE_F16, stream);
     if (rc != FBB_OK) return rc;
-    rc = launch_linear(y, d.qkv_w, qkv, d.qkv_b, nullptr, nullptr, T, 3 * C, C, C, C, 3 * C, 0, FBB_EPI_NONE, d.acc_main, stream);
+    rc = launch_linear(y, d.qkv_w, qkv, d.qkv_b, nullptr, nullptr, T, 3 * C, C, C, C, 3 * C, 0, FBB_EPI_NONE, d.acc_main, stream, true);
     if (rc != FBB_OK) return rc;
     // q, k, v: the three [B, N, H, 64] views of the packed [B, N, 3, H, 64] buffer
     const int64_t qs[3] = {(int64_t)N * 3 * C, 3 * C, 64}, os[3] = {(int64_t)N * C, C, 64};
@@ -59,17 +59,17 @@ static int run_block(const fbb_block_desc& d, const fbb_block_desc* next, bool y
     rc = launch_flash64(q, q + C, q + 2 * C, o, B, N, d.heads, qs, qs, qs, os, d.scale, d.flash_variant, ws, ws_bytes, stream);
     if (rc != FBB_OK) return rc;
     rc = launch_linear_layernorm(o, d.proj_w, x, d.proj_b, x, d.gamma1, T, C, C, C, C, C, C, FBB_EPI_NONE, d.acc_main, d.ln2_w, d.ln2_b, d.eps2, y, C,
-                                 counter, stream);
+                                 counter, stream, true);
     if (rc != FBB_OK) return rc;
     if (d.mlp == FBB_MLP_SWIGLU)
-        rc = launch_linear(y, d.fc1_w, h, d.fc1_b, nullptr, nullptr, T, 2 * d.hidden, C, C, C, d.hidden, 0, FBB_EPI_SWIGLU, d.acc_main, stream);
+        rc = launch_linear(y, d.fc1_w, h, d.fc1_b, nullptr, nullptr, T, 2 * d.hidden, C, C, C, d.hidden, 0, FBB_EPI_SWIGLU, d.acc_main, stream, true);
     else
-        rc = launch_linear(y, d.fc1_w, h, d.fc1_b, nullptr, nullptr, T, d.hidden, C, C, C, d.hidden, 0, FBB_EPI_GELU, d.acc_main, stream);
+        rc = launch_linear(y, d.fc1_w, h, d.fc1_b, nullptr, nullptr, T, d.hidden, C, C, C, d.hidden, 0, FBB_EPI_GELU, d.acc_main, stream, true);
     if (rc != FBB_OK) return rc;
     if (next != nullptr)
         return launch_linear_layernorm(h, d.fc2_w, x, d.fc2_b, x, d.gamma2, T, C, d.hidden, d.hidden, d.hidden, C, C, FBB_EPI_NONE, d.acc_fc2, next->ln1_w,
-                                       next->ln1_b, next->eps1, y, C, counter, stream);
-    return launch_linear(h, d.fc2_w, x, d.fc2_b, x, d.gamma2, T, C, d.hidden, d.hidden, d.hidden, C, C, FBB_EPI_NONE, d.acc_fc2, stream);
+                                       next->ln1_b, next->eps1, y, C, counter, stream, true);
+    return launch_linear(h, d.fc2_w, x, d.fc2_b, x, d.gamma2, T, C, d.hidden, d.hidden, d.hidden, C, C, FBB_EPI_NONE, d.acc_fc2, stream, true);
 }
 
 int stack_launches(const fbb_block_desc* d, int n_blocks, int64_t tokens) {

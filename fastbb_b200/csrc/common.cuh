@@ -175,6 +175,43 @@ __device__ __forceinline__ void tma_store_4d(const void* map, uint32_t src, int 
 __device__ __forceinline__ void stmatrix_x4(uint32_t addr, uint32_t r0, uint32_t r1, uint32_t r2, uint32_t r3) {
     asm volatile("stmatrix.sync.aligned.m8n8.x4.shared.b16 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(r0), "r"(r1), "r"(r2), "r"(r3) : "memory");
 }
+// Announce `bytes` on the barrier (0: not at all) and load one box of each of two tensors, by one elected lane of a converged warp.
+__device__ __forceinline__ void tma_load_2d_two_warp(uint32_t bar, uint32_t bytes, uint32_t dst0, const void* map0, int x0, int y0, uint32_t dst1,
+                                                     const void* map1, int x1, int y1) {
+    asm volatile(
+        "{\n\t"
+        ".reg .pred p, q;\n\t"
+        "setp.ne.b32 p, %1, 0;\n\t"
+        "elect.sync _|q, 0xFFFFFFFF;\n\t"
+        "and.pred p, p, q;\n\t"
+        "@p mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n\t"
+        "@q cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%2], [%3, {%4, %5}], [%0];\n\t"
+        "@q cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%6], [%7, {%8, %9}], [%0];\n\t"
+        "}\n"
+        ::"r"(bar), "r"(bytes), "r"(dst0), "l"(map0), "r"(x0), "r"(y0), "r"(dst1), "l"(map1), "r"(x1), "r"(y1)
+        : "memory");
+}
+__device__ __forceinline__ void tma_load_2d_warp(uint32_t dst, const void* map, uint32_t bar, int x, int y) {
+    asm volatile(
+        "{\n\t"
+        ".reg .pred q;\n\t"
+        "elect.sync _|q, 0xFFFFFFFF;\n\t"
+        "@q cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];\n\t"
+        "}\n"
+        ::"r"(dst), "l"(map), "r"(bar), "r"(x), "r"(y)
+        : "memory");
+}
+__device__ __forceinline__ void tma_load_4d_expect_warp(uint32_t dst, const void* map, uint32_t bar, uint32_t bytes, int c0, int c1, int c2, int c3) {
+    asm volatile(
+        "{\n\t"
+        ".reg .pred q;\n\t"
+        "elect.sync _|q, 0xFFFFFFFF;\n\t"
+        "@q mbarrier.arrive.expect_tx.shared::cta.b64 _, [%2], %7;\n\t"
+        "@q cp.async.bulk.tensor.4d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5, %6}], [%2];\n\t"
+        "}\n"
+        ::"r"(dst), "l"(map), "r"(bar), "r"(c0), "r"(c1), "r"(c2), "r"(c3), "r"(bytes)
+        : "memory");
+}
 __device__ __forceinline__ void bulk_commit() { asm volatile("cp.async.bulk.commit_group;" ::: "memory"); }
 // Until the bulk stores committed by this thread have finished READING shared memory (the buffer may be rewritten).
 __device__ __forceinline__ void bulk_wait_read_all() { asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory"); }
@@ -286,29 +323,95 @@ __host__ __device__ constexpr uint32_t make_idesc_f16(int M, int N, bool acc_f32
 }
 
 
-// Warp-collective forms: every lane of a converged warp executes the call, one elected lane issues the instruction.
-// Keeping the issuing code warp-uniform lets the compiler hold descriptors and addresses in uniform registers, which is
-// what keeps the per-instruction issue cost of a long UMMA sequence low.
-__device__ __forceinline__ void umma_ss_warp(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
+// Warp-collective forms: every lane of a converged warp executes the call, ONE elected lane issues all of its instructions.
+// Keeping the issuing code warp-uniform lets the compiler hold descriptors and addresses in uniform registers; electing once
+// per block and not per instruction is what keeps the issue cost low (measured: 433 clocks per k-block for a ready wait, four
+// separately elected UMMAs and a commit; a producer lane inside an ordinary divergent branch 396 clocks per pair of loads).
+
+// One 64-element k-block of K-major operands: four K16 steps, 32 bytes apart in both tiles, then a commit to `bar`.
+__device__ __forceinline__ void umma_kblock_commit_warp(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accumulate, uint32_t bar) {
     asm volatile(
         "{\n\t"
         ".reg .pred p, q;\n\t"
-        "elect.sync _|q, 0xFFFFFFFF;\n\t"
+        ".reg .b64 a1, a2, a3, b1, b2, b3;\n\t"
+        "add.s64 a1, %1, 2;\n\t"
+        "add.s64 b1, %2, 2;\n\t"
+        "add.s64 a2, %1, 4;\n\t"
+        "add.s64 b2, %2, 4;\n\t"
+        "add.s64 a3, %1, 6;\n\t"
+        "add.s64 b3, %2, 6;\n\t"
         "setp.ne.b32 p, %4, 0;\n\t"
+        "elect.sync _|q, 0xFFFFFFFF;\n\t"
         "@q tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t"
+        "@q tcgen05.mma.cta_group::1.kind::f16 [%0], a1, b1, %3, 1;\n\t"
+        "@q tcgen05.mma.cta_group::1.kind::f16 [%0], a2, b2, %3, 1;\n\t"
+        "@q tcgen05.mma.cta_group::1.kind::f16 [%0], a3, b3, %3, 1;\n\t"
+        "@q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%5];\n\t"
         "}\n"
-        ::"r"(d_tmem), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
+        ::"r"(d_tmem), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate), "r"(bar)
         : "memory");
 }
-__device__ __forceinline__ void umma_ts_warp(uint32_t d_tmem, uint32_t a_tmem, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
+// The same with commits to two barriers, accumulator overwritten (the Q K^T of one key block).
+__device__ __forceinline__ void umma_kblock_commit2_warp(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accumulate, uint32_t bar0,
+                                                         uint32_t bar1) {
     asm volatile(
         "{\n\t"
         ".reg .pred p, q;\n\t"
-        "elect.sync _|q, 0xFFFFFFFF;\n\t"
+        ".reg .b64 a1, a2, a3, b1, b2, b3;\n\t"
+        "add.s64 a1, %1, 2;\n\t"
+        "add.s64 b1, %2, 2;\n\t"
+        "add.s64 a2, %1, 4;\n\t"
+        "add.s64 b2, %2, 4;\n\t"
+        "add.s64 a3, %1, 6;\n\t"
+        "add.s64 b3, %2, 6;\n\t"
         "setp.ne.b32 p, %4, 0;\n\t"
-        "@q tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t"
+        "elect.sync _|q, 0xFFFFFFFF;\n\t"
+        "@q tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t"
+        "@q tcgen05.mma.cta_group::1.kind::f16 [%0], a1, b1, %3, 1;\n\t"
+        "@q tcgen05.mma.cta_group::1.kind::f16 [%0], a2, b2, %3, 1;\n\t"
+        "@q tcgen05.mma.cta_group::1.kind::f16 [%0], a3, b3, %3, 1;\n\t"
+        "@q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%5];\n\t"
+        "@q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%6];\n\t"
         "}\n"
-        ::"r"(d_tmem), "r"(a_tmem), "l"(bdesc), "r"(idesc), "r"(accumulate)
+        ::"r"(d_tmem), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate), "r"(bar0), "r"(bar1)
+        : "memory");
+}
+// A from tensor memory (8 columns per K16 step), B MN-major (2048 bytes per step): eight steps and commits to two barriers.
+__device__ __forceinline__ void umma_ts8_commit2_warp(uint32_t d_tmem, uint32_t a_tmem, uint64_t bdesc, uint32_t idesc, uint32_t accumulate, uint32_t bar0,
+                                                      uint32_t bar1) {
+    asm volatile(
+        "{\n\t"
+        ".reg .pred p, q;\n\t"
+        ".reg .b32 a1, a2, a3, a4, a5, a6, a7;\n\t"
+        ".reg .b64 b1, b2, b3, b4, b5, b6, b7;\n\t"
+        "add.u32 a1, %1, 8;\n\t"
+        "add.s64 b1, %2, 128;\n\t"
+        "add.u32 a2, %1, 16;\n\t"
+        "add.s64 b2, %2, 256;\n\t"
+        "add.u32 a3, %1, 24;\n\t"
+        "add.s64 b3, %2, 384;\n\t"
+        "add.u32 a4, %1, 32;\n\t"
+        "add.s64 b4, %2, 512;\n\t"
+        "add.u32 a5, %1, 40;\n\t"
+        "add.s64 b5, %2, 640;\n\t"
+        "add.u32 a6, %1, 48;\n\t"
+        "add.s64 b6, %2, 768;\n\t"
+        "add.u32 a7, %1, 56;\n\t"
+        "add.s64 b7, %2, 896;\n\t"
+        "setp.ne.b32 p, %4, 0;\n\t"
+        "elect.sync _|q, 0xFFFFFFFF;\n\t"
+        "@q tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t"
+        "@q tcgen05.mma.cta_group::1.kind::f16 [%0], [a1], b1, %3, 1;\n\t"
+        "@q tcgen05.mma.cta_group::1.kind::f16 [%0], [a2], b2, %3, 1;\n\t"
+        "@q tcgen05.mma.cta_group::1.kind::f16 [%0], [a3], b3, %3, 1;\n\t"
+        "@q tcgen05.mma.cta_group::1.kind::f16 [%0], [a4], b4, %3, 1;\n\t"
+        "@q tcgen05.mma.cta_group::1.kind::f16 [%0], [a5], b5, %3, 1;\n\t"
+        "@q tcgen05.mma.cta_group::1.kind::f16 [%0], [a6], b6, %3, 1;\n\t"
+        "@q tcgen05.mma.cta_group::1.kind::f16 [%0], [a7], b7, %3, 1;\n\t"
+        "@q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%5];\n\t"
+        "@q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%6];\n\t"
+        "}\n"
+        ::"r"(d_tmem), "r"(a_tmem), "l"(bdesc), "r"(idesc), "r"(accumulate), "r"(bar0), "r"(bar1)
         : "memory");
 }
 __device__ __forceinline__ void umma_commit_warp(uint32_t bar) {
@@ -335,6 +438,17 @@ __device__ __forceinline__ void cluster_sync_all() {
     asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
     asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
+__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
+// The address in the shared memory of CTA `rank` of this cluster of what `addr` is in this CTA, and a 16-byte store there.
+__device__ __forceinline__ uint32_t map_cluster(uint32_t addr, uint32_t rank) {
+    uint32_t r;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(rank));
+    return r;
+}
+__device__ __forceinline__ void st_cluster_16(uint32_t addr, uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
+    asm volatile("st.shared::cluster.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(a), "r"(b), "r"(c), "r"(d) : "memory");
+}
 // Arrive (count 1) on the barrier at the same shared-memory offset in CTA `rank` of the cluster.
 __device__ __forceinline__ void mbar_arrive_remote(uint32_t bar, uint32_t rank) {
     asm volatile(
@@ -344,14 +458,6 @@ __device__ __forceinline__ void mbar_arrive_remote(uint32_t bar, uint32_t rank) 
         "mbarrier.arrive.release.cluster.shared::cluster.b64 _, [ra];\n\t"
         "}\n"
         ::"r"(bar), "r"(rank)
-        : "memory");
-}
-// TMA tile load of a CTA pair member: data lands in this CTA's shared memory, the byte count is credited to the LEADER's
-// barrier (same offset, cluster rank 0: the CTA-rank bit of the shared::cluster address cleared).
-__device__ __forceinline__ void tma_load_2d_pair(uint32_t dst, const void* map, uint32_t bar, int c0, int c1) {
-    asm volatile(
-        "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
-        ::"r"(dst), "l"(map), "r"(bar & 0xFEFFFFFFu), "r"(c0), "r"(c1)
         : "memory");
 }
 template <int NCOLS>
@@ -365,15 +471,78 @@ template <int NCOLS>
 __device__ __forceinline__ void tmem_dealloc_pair(uint32_t taddr) {
     asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(taddr), "n"(NCOLS) : "memory");
 }
-__device__ __forceinline__ void umma_ss_pair_warp(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
+// One 64-element k-block of the pair's tile (see umma_kblock_commit_warp); the commit arrives at `bar` in the CTAs of `mask`.
+__device__ __forceinline__ void umma_kblock_commit_pair_warp(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accumulate,
+                                                             uint32_t bar, uint32_t mask) {
     asm volatile(
         "{\n\t"
         ".reg .pred p, q;\n\t"
-        "elect.sync _|q, 0xFFFFFFFF;\n\t"
+        ".reg .b16 m;\n\t"
+        ".reg .b64 a1, a2, a3, b1, b2, b3;\n\t"
+        "add.s64 a1, %1, 2;\n\t"
+        "add.s64 b1, %2, 2;\n\t"
+        "add.s64 a2, %1, 4;\n\t"
+        "add.s64 b2, %2, 4;\n\t"
+        "add.s64 a3, %1, 6;\n\t"
+        "add.s64 b3, %2, 6;\n\t"
+        "cvt.u16.u32 m, %6;\n\t"
         "setp.ne.b32 p, %4, 0;\n\t"
+        "elect.sync _|q, 0xFFFFFFFF;\n\t"
         "@q tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t"
+        "@q tcgen05.mma.cta_group::2.kind::f16 [%0], a1, b1, %3, 1;\n\t"
+        "@q tcgen05.mma.cta_group::2.kind::f16 [%0], a2, b2, %3, 1;\n\t"
+        "@q tcgen05.mma.cta_group::2.kind::f16 [%0], a3, b3, %3, 1;\n\t"
+        "@q tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%5], m;\n\t"
+        "}\n"
+        ::"r"(d_tmem), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate), "r"(bar), "r"(mask)
+        : "memory");
+}
+// The four K16 steps alone.
+__device__ __forceinline__ void umma_kblock_pair_warp(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
+    asm volatile(
+        "{\n\t"
+        ".reg .pred p, q;\n\t"
+        ".reg .b64 a1, a2, a3, b1, b2, b3;\n\t"
+        "add.s64 a1, %1, 2;\n\t"
+        "add.s64 b1, %2, 2;\n\t"
+        "add.s64 a2, %1, 4;\n\t"
+        "add.s64 b2, %2, 4;\n\t"
+        "add.s64 a3, %1, 6;\n\t"
+        "add.s64 b3, %2, 6;\n\t"
+        "setp.ne.b32 p, %4, 0;\n\t"
+        "elect.sync _|q, 0xFFFFFFFF;\n\t"
+        "@q tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t"
+        "@q tcgen05.mma.cta_group::2.kind::f16 [%0], a1, b1, %3, 1;\n\t"
+        "@q tcgen05.mma.cta_group::2.kind::f16 [%0], a2, b2, %3, 1;\n\t"
+        "@q tcgen05.mma.cta_group::2.kind::f16 [%0], a3, b3, %3, 1;\n\t"
         "}\n"
         ::"r"(d_tmem), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
+        : "memory");
+}
+// tma_load_2d_two_warp for a pair member: data lands in this CTA's shared memory, the bytes are credited to the leader's barrier.
+__device__ __forceinline__ void tma_load_2d_two_pair_warp(uint32_t bar, uint32_t bytes, uint32_t dst0, const void* map0, int x0, int y0, uint32_t dst1,
+                                                          const void* map1, int x1, int y1) {
+    asm volatile(
+        "{\n\t"
+        ".reg .pred p, q;\n\t"
+        "setp.ne.b32 p, %1, 0;\n\t"
+        "elect.sync _|q, 0xFFFFFFFF;\n\t"
+        "and.pred p, p, q;\n\t"
+        "@p mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n\t"
+        "@q cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%2], [%3, {%4, %5}], [%10];\n\t"
+        "@q cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%6], [%7, {%8, %9}], [%10];\n\t"
+        "}\n"
+        ::"r"(bar), "r"(bytes), "r"(dst0), "l"(map0), "r"(x0), "r"(y0), "r"(dst1), "l"(map1), "r"(x1), "r"(y1), "r"(bar & 0xFEFFFFFFu)
+        : "memory");
+}
+__device__ __forceinline__ void tma_load_2d_pair_warp(uint32_t dst, const void* map, uint32_t bar, int x, int y) {
+    asm volatile(
+        "{\n\t"
+        ".reg .pred q;\n\t"
+        "elect.sync _|q, 0xFFFFFFFF;\n\t"
+        "@q cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];\n\t"
+        "}\n"
+        ::"r"(dst), "l"(map), "r"(bar & 0xFEFFFFFFu), "r"(x), "r"(y)
         : "memory");
 }
 // Arrive on the barrier at this offset in BOTH CTAs of the pair once the UMMAs issued so far have completed.

@@ -525,12 +525,7 @@ flash64_umma_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
         auto issue_qk = [&](int it, int s, bool last) {
             const uint64_t qd = qd0 + (uint64_t)((it & 1) * (2 * kTileBytes >> 4));
             const uint64_t kd = kd0 + (uint64_t)(s * (kTileBytes >> 4));
-            umma_ss_warp(dS, qd, kd, idesc_qk, 0u);
-            umma_ss_warp(dS, qd + 2u, kd + 2u, idesc_qk, 1u);
-            umma_ss_warp(dS, qd + 4u, kd + 4u, idesc_qk, 1u);
-            umma_ss_warp(dS, qd + 6u, kd + 6u, idesc_qk, 1u);
-            umma_commit_warp(s_full(t));
-            umma_commit_warp(k_empty(s));
+            umma_kblock_commit2_warp(dS, qd, kd, idesc_qk, 0u, s_full(t), k_empty(s));
             if (last) umma_commit_warp(q_empty(it & 1));  // this buffer may be loaded again
         };
         int it = 0, kb = 0, kb1 = 0;
@@ -584,11 +579,7 @@ flash64_umma_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
             tc_fence_after();
             FBB_TRACE(2 + t, g, 1);
             const uint64_t vd = vd0 + (uint64_t)(s * (kTileBytes >> 4));
-            umma_ts_warp(dO, aP, vd, idesc_pv, first ? 0u : 1u);
-#pragma unroll
-            for (int k = 1; k < 8; ++k) umma_ts_warp(dO, aP + 8u * k, vd + 128u * k, idesc_pv, 1u);
-            umma_commit_warp(pv_done(t));
-            umma_commit_warp(v_empty(s));
+            umma_ts8_commit2_warp(dO, aP, vd, idesc_pv, first ? 0u : 1u, pv_done(t), v_empty(s));
             FBB_TRACE(2 + t, g, 2);
             if (!have_next) break;
             it = nit;

@@ -20,6 +20,7 @@
 // the plain 256-column form cuts the tiles of a partly filled second wave into 128- or 64-column slices (narrow_tail).
 #include "common.cuh"
 #include <cstdlib>
+#include <mutex>
 
 #include "internal.h"
 
@@ -198,8 +199,8 @@ linear_umma_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_cons
     grid_launch_dependents();
 
     if (warp == 0) {
-        // ------------------------------------------------------------------ TMA producer
-        if (lane == 0) {
+        // ------------------------------------------------------------------ TMA producer (the whole warp, one elected lane issues)
+        {
             int s = 0;
             uint32_t ph = 0;
             bool ok = true;
@@ -208,31 +209,22 @@ linear_umma_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_cons
                 item_at(item, m0, n0, w);
                 const int nt = n0 / kOutCols;
                 for (int kb = 0; kb < num_kb; ++kb) {
-                    if (!mbar_wait(empty_bar(s), ph ^ 1u, s_abort, DEV_TIMEOUT_SMEM_EMPTY, s)) { ok = false; break; }
+                    if (__all_sync(0xffffffffu, mbar_wait(empty_bar(s), ph ^ 1u, s_abort, DEV_TIMEOUT_SMEM_EMPTY, s)) == 0) { ok = false; break; }
                     const uint32_t sa = base + s * S::kStageBytes;
                     const uint32_t sb = sa + S::kABytes;
                     if constexpr (CTA2) {
                         // the leader's barrier collects the bytes of both CTAs; each CTA loads its own A rows and its half of
                         // the W rows (SwiGLU: the leader the x1 rows, the peer the matching x2 rows)
-                        if (rank == 0) mbar_arrive_expect_tx(full_bar(s), 2 * S::kStageBytes);
-                        tma_load_2d_pair(sa, &tmap_a, full_bar(s), kb * BK, m0);
                         const int wrow = SWIGLU ? (rank == 0 ? nt * (BN / 2) : g.N / 2 + nt * (BN / 2)) : nt * BN + (int)rank * (BN / 2);
-                        tma_load_2d_pair(sb, &tmap_w, full_bar(s), kb * BK, wrow);
+                        tma_load_2d_two_pair_warp(full_bar(s), rank == 0 ? 2u * S::kStageBytes : 0u, sa, &tmap_a, kb * BK, m0, sb, &tmap_w, kb * BK, wrow);
                     } else if (kNarrowOk && w != BN) {
                         // a slice: its W rows in 64-row boxes, laid out like the first rows of a whole tile's box
-                        mbar_arrive_expect_tx(full_bar(s), (uint32_t)(S::kABytes + w * BK * 2));
-                        tma_load_2d(sa, &tmap_a, full_bar(s), kb * BK, m0);
-                        for (int r = 0; r < w; r += 64) tma_load_2d(sb + (uint32_t)(r * BK * 2), &tmap_wn, full_bar(s), kb * BK, n0 + r);
+                        tma_load_2d_two_warp(full_bar(s), (uint32_t)(S::kABytes + w * BK * 2), sa, &tmap_a, kb * BK, m0, sb, &tmap_wn, kb * BK, n0);
+                        for (int r = 64; r < w; r += 64) tma_load_2d_warp(sb + (uint32_t)(r * BK * 2), &tmap_wn, full_bar(s), kb * BK, n0 + r);
                     } else {
-                        mbar_arrive_expect_tx(full_bar(s), S::kStageBytes);
-                        tma_load_2d(sa, &tmap_a, full_bar(s), kb * BK, m0);
-                        if (SWIGLU) {
-                            // x1 rows [nt*BN/2, +BN/2) and the matching x2 rows, offset by N/2
-                            tma_load_2d(sb, &tmap_w, full_bar(s), kb * BK, nt * (BN / 2));
-                            tma_load_2d(sb + S::kBBytes / 2, &tmap_w, full_bar(s), kb * BK, g.N / 2 + nt * (BN / 2));
-                        } else {
-                            tma_load_2d(sb, &tmap_w, full_bar(s), kb * BK, nt * BN);
-                        }
+                        // SwiGLU: x1 rows [nt*BN/2, +BN/2) and the matching x2 rows, offset by N/2
+                        tma_load_2d_two_warp(full_bar(s), S::kStageBytes, sa, &tmap_a, kb * BK, m0, sb, &tmap_w, kb * BK, SWIGLU ? nt * (BN / 2) : nt * BN);
+                        if (SWIGLU) tma_load_2d_warp(sb + S::kBBytes / 2, &tmap_w, full_bar(s), kb * BK, g.N / 2 + nt * (BN / 2));
                     }
                     if (++s == kStages) { s = 0; ph ^= 1u; }
                 }
@@ -264,15 +256,9 @@ linear_umma_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_cons
                 const uint64_t adesc = adesc0 + (uint64_t)(s * (S::kStageBytes >> 4));
                 const uint64_t bdesc = adesc + (uint64_t)(S::kABytes >> 4);
                 if constexpr (CTA2) {
-                    umma_ss_pair_warp(d_tmem, adesc, bdesc, idesc, kb != 0 ? 1u : 0u);
-#pragma unroll
-                    for (int k = 1; k < BK / 16; ++k) umma_ss_pair_warp(d_tmem, adesc + 2u * k, bdesc + 2u * k, idesc, 1u);
-                    umma_commit_pair_warp(empty_bar(s));  // frees the stage in both CTAs
+                    umma_kblock_commit_pair_warp(d_tmem, adesc, bdesc, idesc, kb != 0 ? 1u : 0u, empty_bar(s), 3u);  // frees the stage in both CTAs
                 } else {
-                    umma_ss_warp(d_tmem, adesc, bdesc, idesc, kb != 0 ? 1u : 0u);
-#pragma unroll
-                    for (int k = 1; k < BK / 16; ++k) umma_ss_warp(d_tmem, adesc + 2u * k, bdesc + 2u * k, idesc, 1u);
-                    umma_commit_warp(empty_bar(s));  // stage reusable once these UMMAs have read it
+                    umma_kblock_commit_warp(d_tmem, adesc, bdesc, idesc, kb != 0 ? 1u : 0u, empty_bar(s));  // stage reusable once these UMMAs have read it
                 }
                 if (++s == kStages) { s = 0; ph ^= 1u; }
             }
@@ -542,20 +528,19 @@ linear_wide_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid
     grid_launch_dependents();
 
     if (warp == 0) {
-        // ------------------------------------------------------------------ TMA producer (one lane in each CTA)
-        if (lane == 0) {
+        // ------------------------------------------------------------------ TMA producer (one warp in each CTA)
+        {
             int s = 0;
             uint32_t ph = 0;
             bool ok = true;
             const int wrow_a = n0 + (int)rank * (g.wa / 2);
             const int wrow_b = n0 + g.wa + (int)rank * (g.wb / 2);
             for (int kb = 0; kb < num_kb; ++kb) {
-                if (!mbar_wait(empty_bar(s), ph ^ 1u, s_abort, DEV_TIMEOUT_SMEM_EMPTY, s)) { ok = false; break; }
+                if (__all_sync(0xffffffffu, mbar_wait(empty_bar(s), ph ^ 1u, s_abort, DEV_TIMEOUT_SMEM_EMPTY, s)) == 0) { ok = false; break; }
                 const uint32_t sa = base + s * g.stage_bytes;
-                if (rank == 0) mbar_arrive_expect_tx(full_bar(s), 2 * g.stage_bytes);  // the leader's barrier counts both CTAs' bytes
-                tma_load_2d_pair(sa, &tmap_a, full_bar(s), kb * BK, m0);
-                tma_load_2d_pair(sa + BM * BK * 2, &tmap_wa, full_bar(s), kb * BK, wrow_a);
-                if (g.wb > 0) tma_load_2d_pair(sa + BM * BK * 2 + g.wa * BK, &tmap_wb, full_bar(s), kb * BK, wrow_b);
+                // the leader's barrier counts both CTAs' bytes
+                tma_load_2d_two_pair_warp(full_bar(s), rank == 0 ? 2u * g.stage_bytes : 0u, sa, &tmap_a, kb * BK, m0, sa + BM * BK * 2, &tmap_wa, kb * BK, wrow_a);
+                if (g.wb > 0) tma_load_2d_pair_warp(sa + BM * BK * 2 + g.wa * BK, &tmap_wb, full_bar(s), kb * BK, wrow_b);
                 if (++s == g.stages) { s = 0; ph ^= 1u; }
             }
             if (!ok) __nanosleep(20000);  // let copies already in flight land before the CTA leaves
@@ -577,13 +562,9 @@ linear_wide_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid
             const uint64_t adesc = adesc0 + (uint64_t)((s * g.stage_bytes) >> 4);
             const uint64_t bdesc_a = adesc + (uint64_t)((BM * BK * 2) >> 4);
             const uint64_t bdesc_b = bdesc_a + (uint64_t)((g.wa * BK) >> 4);
-#pragma unroll
-            for (int k = 0; k < BK / 16; ++k) {
-                const uint32_t accumulate = (kb != 0 || k != 0) ? 1u : 0u;
-                umma_ss_pair_warp(d_a, adesc + 2u * k, bdesc_a + 2u * k, idesc_a, accumulate);
-                if (g.wb > 0) umma_ss_pair_warp(d_b, adesc + 2u * k, bdesc_b + 2u * k, idesc_b, accumulate);
-            }
-            umma_commit_pair_mask_warp(empty_bar(s), 3u << crank);  // frees the stage in both CTAs (the leader's rank is even)
+            // both accumulators in turn per K16 step would read A twice as close together, but costs an election each: whole k-blocks
+            if (g.wb > 0) umma_kblock_pair_warp(d_b, adesc, bdesc_b, idesc_b, kb != 0 ? 1u : 0u);
+            umma_kblock_commit_pair_warp(d_a, adesc, bdesc_a, idesc_a, kb != 0 ? 1u : 0u, empty_bar(s), 3u << crank);  // frees the stage in both CTAs (the leader's rank is even)
             if (++s == g.stages) { s = 0; ph ^= 1u; }
         }
         if (ok) umma_commit_pair_mask_warp(tfull_bar, 3u << crank);  // both CTAs' accumulators complete
@@ -874,6 +855,309 @@ linear_wide_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid
     }
 }
 
+// ---------------------------------------------------------------------------------------------------------------------
+// Split form: the K loop of a 128 x `bn` tile is shared by the S CTAs of a cluster (1, 2, 4 or 8), for launches whose tiles do
+// not fill the SMs (an image or a few through a small model; the K = 4C layers of a larger one). Such a launch lasts as long
+// as ONE tile: a k-block takes its SM 200 - 400 clocks whatever the tile's width, and ViT-S's fc2 has 24 of them. Each CTA
+// multiplies its share of the k-blocks and sends the fp32 partial tile row by row into the shared memory of the CTA that
+// finishes that row (128 / S rows each); after one cluster barrier every CTA adds the S partials of its rows in rank order
+// (the same result on every run), then bias, GELU, residual. Sending, not fetching: remote stores wait for nothing, while
+// fetching the partials measured 1400 (bn = 32) to 4300 clocks (bn = 128) and needed a second barrier before the CTAs could
+// leave. Eight columns per thread: residual and output move in 16-byte pieces of consecutive lanes, without staging.
+constexpr int kSplitMaxGroups = 4;  // eight-column groups per thread: (128 / S) * (bn / 8) <= 4 * 256
+
+struct SplitArgs {
+    __half* C;
+    const __half* bias;
+    const __half* res;
+    const __half* gamma;
+    int M, N, K;
+    int64_t ldc, ldr;
+    int act, acc_f16;
+    int bn, tiles_n;           // tile width (32, 64 or 128); tiles per row of tiles
+    int stages, stage_bytes;   // operand ring: A tile (16 KB) | bn rows of W
+    int w_early;               // W was complete before the previous launch started: load it ahead of the dependency wait
+};
+
+struct SplitSmem {  // ring | partials [S][128 / S rows][bn floats + 16 bytes] | barriers
+    static constexpr int kMaxStages = 8;
+    static constexpr int kNumBars = 2 * kMaxStages + 1;
+    static constexpr int kTailBytes = kNumBars * 8 + 16;
+    static constexpr int kMaxDynamic = 227 * 1024;
+    static constexpr int stage_bytes(int bn) { return (BM + bn) * BK * 2; }
+    static constexpr int partial_bytes(int bn) { return BM * (bn * 4 + 16); }  // row stride / 16 is odd: no bank conflicts down a column
+};
+
+template <int S>
+__global__ void __launch_bounds__(kGemmThreads, 1)
+linear_split_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_w, const SplitArgs g) {
+    using SS = SplitSmem;
+    constexpr int kRows = BM / S;
+    const uint32_t rank = S > 1 ? cluster_ctarank() : 0u;
+    const int tile = (int)blockIdx.x / S;
+    const int m0 = (tile / g.tiles_n) * BM, n0 = (tile % g.tiles_n) * g.bn;
+    extern __shared__ uint8_t smem_raw[];
+    const uint32_t raw = smem_u32(smem_raw);
+    const uint32_t base = (raw + 1023u) & ~1023u;
+    uint8_t* gen = smem_raw + (base - raw);
+    const int part_off = g.stages * g.stage_bytes, part_stride = g.bn * 4 + 16, bar_off = part_off + BM * part_stride;
+    const uint32_t bar0 = base + (uint32_t)bar_off;
+    auto full_bar = [&](int s) { return bar0 + 8u * s; };
+    auto empty_bar = [&](int s) { return bar0 + 8u * (SS::kMaxStages + s); };
+    const uint32_t tfull_bar = bar0 + 8u * (2 * SS::kMaxStages);
+    volatile uint32_t* s_tmem = reinterpret_cast<volatile uint32_t*>(gen + bar_off + SS::kNumBars * 8);
+    volatile int* s_abort = reinterpret_cast<volatile int*>(gen + bar_off + SS::kNumBars * 8 + 4);
+
+    const int warp = threadIdx.x >> 5;
+    const int lane = threadIdx.x & 31;
+    const int num_kb = (g.K + BK - 1) / BK;
+    const int kb0 = num_kb * (int)rank / S, nkb = num_kb * ((int)rank + 1) / S - kb0;  // this CTA's k-blocks (at least one)
+
+    if (threadIdx.x == 0) {
+        for (int s = 0; s < g.stages; ++s) {
+            mbar_init(full_bar(s), 1);
+            mbar_init(empty_bar(s), 1);
+        }
+        mbar_init(tfull_bar, 1);
+        *s_abort = 0;
+        fence_barrier_init();
+        if (g.w_early) {
+            for (int i = 0; i < g.stages && i < nkb; ++i) {
+                mbar_arrive_expect_tx(full_bar(i), (uint32_t)g.stage_bytes);
+                tma_load_2d(base + i * g.stage_bytes + BM * BK * 2, &tmap_w, full_bar(i), (kb0 + i) * BK, n0);
+            }
+        }
+        tma_prefetch_desc(&tmap_a);
+        tma_prefetch_desc(&tmap_w);
+    }
+    if (warp == 1) {
+        __syncwarp();
+        tmem_alloc<128>(smem_u32(const_cast<uint32_t*>(s_tmem)));
+        tmem_relinquish();
+    }
+    tc_fence_before();
+    __syncthreads();
+    if constexpr (S > 1) cluster_arrive();  // this CTA is running: the others may store to its shared memory (they wait for it further down)
+    tc_fence_after();
+    const uint32_t tmem_base = *s_tmem;
+    grid_dependency_wait();
+    grid_launch_dependents();
+
+    // the rows of the tile that this CTA finishes, and this thread's eight-column groups of them (256 threads are a multiple of
+    // the groups per row: a thread's groups share their columns)
+    const int per_row = g.bn >> 3, shift = 31 - __clz(per_row), groups = kRows * per_row;
+    const int et = (int)threadIdx.x - 64;
+    const int gcol = (et & (per_row - 1)) * 8, grow0 = et >> shift, grow_step = kEpiThreads >> shift;
+    const int col = n0 + gcol;
+    uint4 rr[kSplitMaxGroups];
+    float bias[8], gamma[8];
+
+    if (warp == 0) {
+        int s = 0;
+        uint32_t ph = 0;
+        bool ok = true;
+        for (int i = 0; i < nkb; ++i) {
+            if (i >= g.stages && !mbar_wait(empty_bar(s), ph ^ 1u, s_abort, DEV_TIMEOUT_SMEM_EMPTY, s)) ok = false;
+            if (__all_sync(0xffffffffu, ok) == 0) { ok = false; break; }
+            const uint32_t sa = base + s * g.stage_bytes;
+            if (g.w_early && i < g.stages) tma_load_2d_warp(sa, &tmap_a, full_bar(s), (kb0 + i) * BK, m0);
+            else tma_load_2d_two_warp(full_bar(s), (uint32_t)g.stage_bytes, sa, &tmap_a, (kb0 + i) * BK, m0, sa + BM * BK * 2, &tmap_w, (kb0 + i) * BK, n0);
+            if (++s == g.stages) { s = 0; ph ^= 1u; }
+        }
+        if (!ok) __nanosleep(20000);  // let copies already in flight land before the CTA leaves
+    } else if (warp == 1) {
+        const uint32_t idesc = make_idesc_f16(BM, g.bn, !g.acc_f16, false, false);
+        constexpr uint64_t desc_hi = make_smem_desc_hi(16, 1024);
+        const uint64_t adesc0 = smem_desc(base, desc_hi);
+        int s = 0;
+        uint32_t ph = 0;
+        bool ok = true;
+        for (int i = 0; i < nkb; ++i) {
+            if (__all_sync(0xffffffffu, mbar_wait(full_bar(s), ph, s_abort, DEV_TIMEOUT_TMA_FULL, s)) == 0) { ok = false; break; }
+            tc_fence_after();
+            const uint64_t adesc = adesc0 + (uint64_t)((s * g.stage_bytes) >> 4);
+            umma_kblock_commit_warp(tmem_base, adesc, adesc + (uint64_t)((BM * BK * 2) >> 4), idesc, i != 0 ? 1u : 0u, empty_bar(s));
+            if (++s == g.stages) { s = 0; ph ^= 1u; }
+        }
+        if (ok) umma_commit_warp(tfull_bar);
+    } else {
+        // residual, bias and LayerScale of this thread's groups, under the main loop
+#pragma unroll
+        for (int i = 0; i < kSplitMaxGroups; ++i) {
+            const int row = m0 + (int)rank * kRows + grow0 + i * grow_step;
+            rr[i] = (g.res != nullptr && et + i * kEpiThreads < groups && row < g.M && col < g.N)
+                        ? *reinterpret_cast<const uint4*>(g.res + (int64_t)row * g.ldr + col) : make_uint4(0u, 0u, 0u, 0u);
+        }
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            bias[j] = (g.bias != nullptr && col < g.N) ? __half2float(g.bias[col + j]) : 0.f;
+            gamma[j] = (g.gamma != nullptr && col < g.N) ? __half2float(g.gamma[col + j]) : 1.f;
+        }
+    }
+    __syncwarp();
+    if constexpr (S > 1) cluster_wait();  // every CTA of the cluster is running
+    if (warp >= 2 && mbar_wait(tfull_bar, 0u, s_abort, DEV_TIMEOUT_TMEM_FULL, 0)) {
+        tc_fence_after();
+        const int quad = warp & 3, trow = quad * 32 + lane, owner = trow / kRows;
+        const uint32_t t_row = tmem_base + ((uint32_t)(quad * 32) << 16);
+        const uint32_t dst = map_cluster(base + (uint32_t)(part_off + ((int)rank * kRows + trow - owner * kRows) * part_stride), (uint32_t)owner);
+        if (m0 + quad * 32 < g.M) {  // (rows of padding are nobody's)
+#pragma unroll 1
+            for (int c0 = ((warp - 2) >> 2) * 32; c0 < g.bn; c0 += 64) {
+                uint32_t r[32];
+                tmem_ld32(t_row + (uint32_t)c0, r);
+                tmem_wait_ld();
+                if (g.acc_f16) {
+#pragma unroll
+                    for (int j = 0; j < 32; ++j) r[j] = __float_as_uint(__half2float(__ushort_as_half((unsigned short)(r[j] & 0xFFFFu))));
+                }
+#pragma unroll
+                for (int j = 0; j < 32; j += 4) st_cluster_16(dst + (uint32_t)((c0 + j) * 4), r[j], r[j + 1], r[j + 2], r[j + 3]);
+            }
+        }
+    }
+    tc_fence_before();
+    __syncwarp();
+    if constexpr (S > 1) {
+        cluster_arrive();
+        cluster_wait();  // the partials of this CTA's rows have arrived; nobody touches another CTA's memory from here on
+    } else {
+        __syncthreads();
+    }
+    if (warp >= 2) {
+        const uint8_t* part = gen + part_off;
+#pragma unroll
+        for (int i = 0; i < kSplitMaxGroups; ++i) {
+            const int lrow = grow0 + i * grow_step, row = m0 + (int)rank * kRows + lrow;
+            if (et + i * kEpiThreads >= groups || row >= g.M || col >= g.N) break;
+            float v[8];
+#pragma unroll
+            for (int k = 0; k < S; ++k) {
+                const float4* p = reinterpret_cast<const float4*>(part + (k * kRows + lrow) * part_stride + gcol * 4);
+                const float4 a = p[0], b = p[1];
+                const float q[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+#pragma unroll
+                for (int j = 0; j < 8; ++j) v[j] = k == 0 ? q[j] : v[j] + q[j];
+            }
+#pragma unroll
+            for (int j = 0; j < 8; ++j) v[j] += bias[j];
+            if (g.act == 1) {
+#pragma unroll
+                for (int j = 0; j < 8; j += 2) {
+                    const float2 y = gelu_erf2(make_float2(v[j], v[j + 1]));
+                    v[j] = y.x;
+                    v[j + 1] = y.y;
+                }
+            }
+            if (g.res != nullptr) {
+                const __half2* rh = reinterpret_cast<const __half2*>(&rr[i]);
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    const float2 rf = __half22float2(rh[j]);
+                    v[2 * j] = fmaf(gamma[2 * j], v[2 * j], rf.x);
+                    v[2 * j + 1] = fmaf(gamma[2 * j + 1], v[2 * j + 1], rf.y);
+                }
+            }
+            *reinterpret_cast<uint4*>(g.C + (int64_t)row * g.ldc + col) = make_uint4(pack_h2(v[0], v[1]), pack_h2(v[2], v[3]), pack_h2(v[4], v[5]), pack_h2(v[6], v[7]));
+        }
+    } else if (warp == 1) {
+        tc_fence_after();  // the epilogue warps' reads of the accumulator are before the barrier
+        tmem_dealloc<128>(tmem_base);
+    }
+}
+
+// Clusters of S CTAs of the split kernel that can be resident at once on the current device (0: cannot be launched).
+template <int S>
+static int split_query_clusters() {
+    int n = 0;
+    if (cudaFuncSetAttribute(linear_split_kernel<S>, cudaFuncAttributeMaxDynamicSharedMemorySize, SplitSmem::kMaxDynamic) == cudaSuccess) {
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3((unsigned)(S * num_sms()));
+        cfg.blockDim = dim3(kGemmThreads);
+        cfg.dynamicSmemBytes = SplitSmem::kMaxDynamic;
+        cudaLaunchAttribute attr[1];
+        attr[0].id = cudaLaunchAttributeClusterDimension;
+        attr[0].val.clusterDim.x = S;
+        attr[0].val.clusterDim.y = 1;
+        attr[0].val.clusterDim.z = 1;
+        cfg.attrs = attr;
+        cfg.numAttrs = 1;
+        if (cudaOccupancyMaxActiveClusters(&n, linear_split_kernel<S>, &cfg) != cudaSuccess) n = 0;
+    }
+    cudaGetLastError();
+    return n;
+}
+struct SplitClusters {
+    int n[4];  // by log2 of the cluster size
+};
+static const SplitClusters& split_max_clusters() {
+    static std::once_flag once[64];
+    static SplitClusters cached[64] = {};
+    int dev = 0;
+    cudaGetDevice(&dev);
+    if (dev < 0 || dev >= 64) dev = 0;
+    std::call_once(once[dev], [dev]() {
+        cached[dev] = SplitClusters{{split_query_clusters<1>(), split_query_clusters<2>(), split_query_clusters<4>(), split_query_clusters<8>()}};
+    });
+    return cached[dev];
+}
+
+// Whether the split form takes tiles of `bn` columns shared by `s` CTAs: one wave, at least one k-block each, no more groups
+// per thread than the kernel holds.
+static bool split_fits(const SplitClusters& most, int64_t M, int N, int K, int bn, int s) {
+    if (!(s == 1 || s == 2 || s == 4 || s == 8) || !(bn == 32 || bn == 64 || bn == 128)) return false;
+    if ((K + BK - 1) / BK < s || (BM / s) * (bn / 8) > kSplitMaxGroups * kEpiThreads) return false;
+    return ((M + BM - 1) / BM) * ((N + bn - 1) / bn) <= most.n[s == 8 ? 3 : s >> 1];
+}
+
+// Time of the split form in us, fitted to measurements on B200 (back-to-back launches with dependent launch): a fixed part
+// per tile width and cluster size (start, the exchange of partials, output) and 0.19 us per k-block of the longest share.
+static double split_cost_us(int K, int bn, int s) {
+    static const double fixed[4][3] = {{2.1, 2.5, 4.0}, {2.7, 3.4, 4.8}, {3.1, 3.8, 6.4}, {3.9, 4.1, 6.4}};  // [log2 s][log2 bn / 32]
+    const int num_kb = (K + BK - 1) / BK;
+    return fixed[s == 8 ? 3 : s >> 1][bn >> 6] + 0.19 * (double)((num_kb + s - 1) / s);
+}
+
+static int launch_split(const void* A, const void* W, const GemmArgs& base, int64_t lda, int64_t ldw, int bn, int s, bool w_early, cudaStream_t stream) {
+    SplitArgs g;
+    g.C = base.C;
+    g.bias = base.bias;
+    g.res = base.res;
+    g.gamma = base.gamma;
+    g.M = base.M;
+    g.N = base.N;
+    g.K = base.K;
+    g.ldc = base.ldc;
+    g.ldr = base.ldr;
+    g.act = base.act;
+    g.acc_f16 = base.acc_f16;
+    g.bn = bn;
+    g.tiles_n = (g.N + bn - 1) / bn;
+    g.stage_bytes = SplitSmem::stage_bytes(bn);
+    const int most = ((g.K + BK - 1) / BK + s - 1) / s;  // k-blocks of the CTA with the most of them
+    int stages = (SplitSmem::kMaxDynamic - 1024 - SplitSmem::kTailBytes - SplitSmem::partial_bytes(bn)) / g.stage_bytes;
+    if (stages > SplitSmem::kMaxStages) stages = SplitSmem::kMaxStages;
+    g.stages = stages < most ? stages : most;
+    g.w_early = w_early ? 1 : 0;
+    CUtensorMap ta, tw;
+    uint64_t dims_a[2] = {(uint64_t)g.K, (uint64_t)g.M};
+    int64_t str_a[2] = {1, lda};
+    uint32_t box_a[2] = {BK, BM};
+    int st = make_tmap_f16(&ta, A, 2, dims_a, str_a, box_a);
+    if (st != FBB_OK) return st;
+    uint64_t dims_w[2] = {(uint64_t)g.K, (uint64_t)g.N};
+    int64_t str_w[2] = {1, ldw};
+    uint32_t box_w[2] = {BK, (uint32_t)bn};
+    st = make_tmap_f16(&tw, W, 2, dims_w, str_w, box_w);
+    if (st != FBB_OK) return st;
+    const unsigned grid = (unsigned)(((g.M + BM - 1) / BM) * g.tiles_n * s);
+    const size_t smem = 1024 + (size_t)g.stages * g.stage_bytes + SplitSmem::partial_bytes(bn) + SplitSmem::kTailBytes;
+    auto kern = s == 8 ? linear_split_kernel<8> : (s == 4 ? linear_split_kernel<4> : (s == 2 ? linear_split_kernel<2> : linear_split_kernel<1>));
+    cudaError_t e = launch_pdl_cluster(kern, dim3(grid), dim3(kGemmThreads), smem, stream, (unsigned)s, ta, tw, g);
+    if (e != cudaSuccess) return fail((int)e, "linear_split_kernel launch: %s", cudaGetErrorString(e));
+    return FBB_OK;
+}
+
 // Clusters of two that can be resident at once for this kernel on the current device (0: pairs cannot be launched).
 template <int BN, bool SWIGLU>
 static int max_pairs() {
@@ -1151,7 +1435,7 @@ int linear_layernorm_launches(int64_t M, int N, int epilogue, bool has_counter) 
 // pairs of a row tile in one cluster) when the shape allows it, otherwise the GEMM followed by the LayerNorm kernel.
 int launch_linear_layernorm(const void* A, const void* W, void* C, const void* bias, const void* res, const void* gamma, int64_t M, int N,
                             int K, int64_t lda, int64_t ldw, int64_t ldc, int64_t ldr, int epilogue, int accumulate, const void* ln_w,
-                            const void* ln_b, float ln_eps, void* y, int64_t ldy, void* counter, cudaStream_t stream) {
+                            const void* ln_b, float ln_eps, void* y, int64_t ldy, void* counter, cudaStream_t stream, bool w_early) {
     if (M == 0) return FBB_OK;
     {
         const int w = fused_layernorm_width(M, N, epilogue, counter != nullptr);
@@ -1186,7 +1470,7 @@ int launch_linear_layernorm(const void* A, const void* W, void* C, const void* b
             return launch_wide(A, W, C, g, lda, ldw, w, stream, ln);
         }
     }
-    const int rc = launch_linear(A, W, C, bias, res, gamma, M, N, K, lda, ldw, ldc, ldr, epilogue, accumulate, stream);
+    const int rc = launch_linear(A, W, C, bias, res, gamma, M, N, K, lda, ldw, ldc, ldr, epilogue, accumulate, stream, w_early);
     if (rc != FBB_OK) return rc;
     return launch_layernorm(C, y, ln_w, ln_b, M, N, ldc, ldy, ln_eps, FBB_DTYPE_F16, FBB_DTYPE_F16, stream);
 }
@@ -1203,7 +1487,7 @@ int linear_max_pairs(int bn) { return bn == 128 ? max_pairs<128, false>() : max_
 
 int launch_linear(const void* A, const void* W, void* C, const void* bias, const void* res, const void* gamma, int64_t M,
                   int N, int K, int64_t lda, int64_t ldw, int64_t ldc, int64_t ldr, int epilogue, int accumulate,
-                  cudaStream_t stream) {
+                  cudaStream_t stream, bool w_early) {
     if (M == 0) return FBB_OK;
     const bool swiglu = epilogue == FBB_EPI_SWIGLU;
     GemmArgs g;
@@ -1287,8 +1571,40 @@ int launch_linear(const void* A, const void* W, void* C, const void* bias, const
             if (2 * items >= wide_pairs && c < best) wide_w = wide_rule_w;
         }
     }
+    // The split form: a candidate where its tiles times its cluster size fit the SMs at once, taken where its time (see
+    // split_cost_us) is below that of the forms above, 2.7 us and 0.9 of the model's units of time. Measured on B200 (us,
+    // without / with): M = 257: N = 384, K = 1536 8.4 / 4.8 (two CTAs per tile of 32 columns), K = 384 5.2 / 3.2 (one);
+    // N = 1152, K = 384 4.4 / 3.2; N = 768, K = 3072 13.2 / 7.5; N = 1024, K = 4096 16.3 / 9.6; M = 1041: N = 768, K = 3072
+    // 14.3 / 10.2, K = 768 6.5 / 4.9; M = 2056, N = 384, K = 1536 10.3 / 7.5.
+    int split_bn = 0, split_s = 0;
+    if (!swiglu && M <= 148 * BM) {
+        const SplitClusters& most = split_max_clusters();
+        const double unit_us = 0.37 * (double)((K + BK - 1) / BK) + 1.0;
+        double split_best = 2.7 + 0.9 * unit_us * best;
+        if (wide_w > 0) {  // a k-block of a wide item takes no less than 0.2 us, and its epilogue overlaps nothing
+            const double kb_us = 0.44 * (double)wide_w / 352.0;
+            split_best = 2.7 + 0.02 * (double)wide_w + (double)((K + BK - 1) / BK) * (kb_us > 0.2 ? kb_us : 0.2);
+        }
+        for (int ks = 1; ks <= 8; ks *= 2) {
+            for (int bn = 32; bn <= 128; bn *= 2) {
+                if (!split_fits(most, M, N, K, bn, ks) || split_cost_us(K, bn, ks) >= split_best) continue;
+                split_best = split_cost_us(K, bn, ks);
+                split_bn = bn;
+                split_s = ks;
+            }
+        }
+    }
     if (const char* f = getenv("FBB_GEMM_FORCE")) {
         wide_w = 0;
+        split_bn = 0;
+        if (f[0] == 'k' && !swiglu) {
+            char* end = nullptr;
+            const int ks = (int)strtol(f + 1, &end, 10), bn = *end == 'x' ? atoi(end + 1) : 0;
+            if (split_fits(split_max_clusters(), M, N, K, bn, ks)) {
+                split_bn = bn;
+                split_s = ks;
+            }
+        }
         if (f[0] == 'w' && !swiglu && wide_max_pairs() > 0) {
             const int w = f[1] == 'a' ? wide_rule_w : atoi(f + 1);  // "wa": the rule's own width, whatever the cost model says
             if (w >= 32 && w <= kWideMaxCols && (w & 31) == 0) wide_w = w;
@@ -1300,6 +1616,7 @@ int launch_linear(const void* A, const void* W, void* C, const void* bias, const
         }
     }
 
+    if (split_bn > 0) return launch_split(A, W, g, lda, ldw, split_bn, split_s, w_early, stream);
     if (wide_w > 0) return launch_wide(A, W, C, g, lda, ldw, wide_w, stream);
 
     CUtensorMap ta, tw;

@@ -69,15 +69,18 @@ int launch_layernorm(const void* x, void* y, const void* w, const void* b, int64
 int launch_layernorm_split(const void* x, const void* w, const void* b, void* patches_out, void* cls_out, void* regs_out, int B, int N, int C,
                            int n_prefix, float eps, int apply_norm, int channel_major, cudaStream_t stream);
 
+// w_early: W (and nothing else) was written before the launch that precedes this one on the stream STARTED, so that its tiles may
+// be loaded ahead of the dependency wait. True inside a run of blocks: every kernel there starts its dependents only after its
+// own wait, so when a GEMM's CTAs start, everything before the launch in front of it is complete, and that launch writes no weights.
 int launch_linear(const void* A, const void* W, void* C, const void* bias, const void* res, const void* gamma, int64_t M,
                   int N, int K, int64_t lda, int64_t ldw, int64_t ldc, int64_t ldr, int epilogue, int accumulate,
-                  cudaStream_t stream);
+                  cudaStream_t stream, bool w_early = false);
 
 // The same followed by y = LayerNorm(C) * ln_w + ln_b (rows of N elements), fused into the GEMM launch when the shape
 // allows. `counter`: 4 bytes of zeroed device memory that every launch leaves zero (needed when M has remainder rows).
 int launch_linear_layernorm(const void* A, const void* W, void* C, const void* bias, const void* res, const void* gamma, int64_t M, int N,
                             int K, int64_t lda, int64_t ldw, int64_t ldc, int64_t ldr, int epilogue, int accumulate, const void* ln_w,
-                            const void* ln_b, float ln_eps, void* y, int64_t ldy, void* counter, cudaStream_t stream);
+                            const void* ln_b, float ln_eps, void* y, int64_t ldy, void* counter, cudaStream_t stream, bool w_early = false);
 
 int linear_layernorm_launches(int64_t M, int N, int epilogue, bool has_counter);  // 1: one fused launch, 2: GEMM then LayerNorm
 

@@ -192,6 +192,32 @@ def test_linear_every_tile_form_matches_oracle(oracle, form, monkeypatch):
     status_ok()
 
 
+@pytest.mark.parametrize("bn", [32, 64, 128])
+@pytest.mark.parametrize("ctas", [1, 2, 4, 8])
+def test_linear_split_form_matches_oracle(oracle, ctas, bn, monkeypatch):
+    """The form whose tiles are shared by the CTAs of a cluster along K: row and column remainders, a ragged last k-block, shares
+    of unequal length, more k-blocks per CTA than the operand ring holds, one row, the residual updated in place."""
+    from fastbb_b200.gemm import linear
+    monkeypatch.setenv("FBB_GEMM_FORCE", f"k{ctas}x{bn}")
+    g = torch.Generator().manual_seed(ctas * 1000 + bn)
+    for M, N, K, act, variant, bias in [(257, 136, 520, None, "f32", True), (129, 200, 1096, "gelu", "f32", True), (1, 64, 512, None, "h", False),
+                                        (128, 8, 8 * 64 * ctas + 72, None, "f32", True), (383, 264, 1024, "gelu", "h", False)]:
+        x = torch.randn(M, K, generator=g).half()
+        w = (torch.randn(N, K, generator=g) / K ** 0.5).half()
+        b = (0.1 * torch.randn(N, generator=g)).half() if bias else None
+        res = torch.randn(M, N, generator=g).half() if act is None else None
+        gam = (0.05 + 0.15 * torch.rand(N, generator=g)).half() if act is None and bias else None
+        out, check = padded((M, N))
+        if res is not None:
+            out.copy_(res)
+        d = lambda t: None if t is None else t.to(dev())  # noqa: E731
+        y = linear(d(x), d(w), d(b), act=act, res=out if res is not None else None, gamma=d(gam), variant=variant, out=out)
+        want = oracle.linear(x, w, b, act=act, res=res, gamma=gam)
+        assert oracle.rel_l2(y.cpu().float(), want) < (TOL_F16 if variant == "h" else TOL_F32), (M, N, K, act)
+        check()
+    status_ok()
+
+
 @pytest.mark.parametrize("M,N,K,act,variant", [(2561, 2000, 136, "gelu", "f32"), (2561, 1848, 72, None, "h"), (6145, 1024, 64, None, "f32"),
                                                 (2600, 2048, 200, None, "f32")])
 def test_linear_last_wave_in_slices_equals_whole_tiles(oracle, M, N, K, act, variant, monkeypatch):
