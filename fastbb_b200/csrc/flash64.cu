@@ -245,7 +245,7 @@ __global__ void __launch_bounds__(128, 16) flash64_side_rows_kernel(const SideAr
                 float acc = 0.f;
 #pragma unroll 2
                 for (int d = 0; d < 8; ++d) {
-                    const uint4 kk = __ldcg(kv + d), qq = __ldg(qv + d);  // K and V stream past L1, which holds the tiled kernel's spills
+                    const uint4 kk = __ldcg(kv + d), qq = __ldg(qv + d);  // K and V stream past L1: each byte is used once
                     const __half2* kh = reinterpret_cast<const __half2*>(&kk);
                     const __half2* qh = reinterpret_cast<const __half2*>(&qq);
 #pragma unroll

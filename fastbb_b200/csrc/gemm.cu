@@ -3,7 +3,7 @@
 // gemm_tn_* kernels of fastbb/fastbb_kernels.cu:323-446 (epilogue order bias -> act -> res + gamma*v, :418-427).
 //
 // K is consumed in 64-element (128-byte) blocks; both operands are K-major, so neither is transposed: nn.Linear's [N, K]
-// weight is exactly the B operand. Three forms, picked per shape by launch_linear's cost model:
+// weight is exactly the B operand. Four forms, picked per shape by launch_linear's cost model:
 //   linear_umma_kernel<BN, SWIGLU, false>  persistent, one CTA per SM, 128 x BN output tiles (cta_group::1)
 //   linear_umma_kernel<BN, SWIGLU, true>   persistent, a pair of CTAs (cluster of two, cta_group::2) on a 256 x BN tile: each
 //                                          CTA stages its 128 rows of A and BN/2 of the W rows, the leader issues UMMAs that
@@ -11,6 +11,8 @@
 //   linear_wide_pair_kernel                one pair per work item of 256 rows x w columns (w <= 512 in two accumulators), not
 //                                          persistent: for shapes with few tiles, where fixed tiles quantise badly; optionally
 //                                          with the LayerNorm of the output rows fused (clusters of up to four pairs)
+//   linear_split_kernel<S>                 one 128 x 32 / 64 / 128 tile per cluster of S CTAs, which share its K loop: for launches
+//                                          whose tiles do not fill the SMs
 // No load is multicast: every CTA fetches its own operands with plain TMA loads; only barrier signals cross a pair.
 //   warp 0      TMA producer: A box [64 x 128] and the W boxes per stage (128-byte swizzle, zero fill outside)
 //   warp 1      UMMA issuer: 4 x tcgen05.mma (K = 16 each) per stage and accumulator
@@ -562,7 +564,7 @@ linear_wide_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid
             const uint64_t adesc = adesc0 + (uint64_t)((s * g.stage_bytes) >> 4);
             const uint64_t bdesc_a = adesc + (uint64_t)((BM * BK * 2) >> 4);
             const uint64_t bdesc_b = bdesc_a + (uint64_t)((g.wa * BK) >> 4);
-            // both accumulators in turn per K16 step would read A twice as close together, but costs an election each: whole k-blocks
+            // one accumulator's whole k-block, then the other's with the commit: two elections per k-block
             if (g.wb > 0) umma_kblock_pair_warp(d_b, adesc, bdesc_b, idesc_b, kb != 0 ? 1u : 0u);
             umma_kblock_commit_pair_warp(d_a, adesc, bdesc_a, idesc_a, kb != 0 ? 1u : 0u, empty_bar(s), 3u << crank);  // frees the stage in both CTAs (the leader's rank is even)
             if (++s == g.stages) { s = 0; ph ^= 1u; }
