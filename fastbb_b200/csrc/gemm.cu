@@ -1579,7 +1579,7 @@ int launch_linear(const void* A, const void* W, void* C, const void* bias, const
     // N = 1152, K = 384 4.4 / 3.2; N = 768, K = 3072 13.2 / 7.5; N = 1024, K = 4096 16.3 / 9.6; M = 1041: N = 768, K = 3072
     // 14.3 / 10.2, K = 768 6.5 / 4.9; M = 2056, N = 384, K = 1536 10.3 / 7.5.
     int split_bn = 0, split_s = 0;
-    if (!swiglu && M <= 148 * BM) {
+    if (!swiglu && ((M + BM - 1) / BM) * tn128 <= sms) {  // (its widest tiles, one CTA each, fit the SMs at once)
         const SplitClusters& most = split_max_clusters();
         const double unit_us = 0.37 * (double)((K + BK - 1) / BK) + 1.0;
         double split_best = 2.7 + 0.9 * unit_us * best;
