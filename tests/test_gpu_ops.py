@@ -473,6 +473,26 @@ def test_flash_peaked_rows_default_scale_and_bhnd_layout(oracle, variant):
     assert oracle.rel_l2(o.cpu().float(), want) < 2e-3
 
 
+@pytest.mark.parametrize("B,N,H", [(1, 17, 3), (1, 129, 2), (2, 385, 6), (3, 1041, 16), (1, 2561, 16)])
+def test_flash_maxima_raised_block_after_block_into_a_strided_output(oracle, B, N, H):
+    """Scores that grow with the key index, so that later blocks (the ragged one too) raise the running maximum by more than the
+    2^8 it may lag, in some rows of a warp and not in others; the output is a strided view whose surroundings must stay."""
+    from fastbb_b200.attention import attention
+    g = torch.Generator().manual_seed(N)
+    q, k, v = (torch.randn(B, N, H, 64, generator=g).half() for _ in range(3))
+    q[:, ::3, :, 0] = 8.0  # every third row sees the ramp: 8 * 8 / 8 = 8 score units, 2^11.5, a block
+    k[..., 0] = (8.0 * (torch.arange(N) // 128)).clamp(max=120).half()[None, :, None]
+    buf = torch.full((B, N + 2, H + 1, 72), CANARY, dtype=torch.float16, device=dev())
+    out = buf[:, 1:N + 1, :H, :64]
+    got = attention(q.to(dev()), k.to(dev()), v.to(dev()), out=out)
+    assert got.data_ptr() == out.data_ptr()
+    want = oracle.attention(q, k, v)
+    assert oracle.rel_l2(out.cpu().float(), want) < 2e-3  # P and O are rounded to fp16 once each: 2 * 2^-11 at most, doubled
+    out.fill_(CANARY)
+    assert torch.all(buf == CANARY), "kernel wrote outside its output"
+    status_ok()
+
+
 @pytest.mark.parametrize("variant", ["ff", "fh", "hh"])
 @pytest.mark.parametrize("N", [4097, 6145, 16385])
 def test_flash_full_size_properties(variant, N):
