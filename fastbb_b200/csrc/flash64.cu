@@ -723,6 +723,8 @@ flash64_umma_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
                     if (g > 0 && !mbar_wait(pv_done(t), (g - 1u) & 1u, s_abort, DEV_TIMEOUT_OTHER, 210 + t)) { ok = false; break; }
                     tc_fence_after();
                     if (done >= 0 && !finish()) { ok = false; break; }
+                    tc_fence_before();  // finish() read O_t, which the P.V that this arrival lets go overwrites
+                    __syncwarp();
                     if (lane == 0) mbar_arrive(p_ready(t));
                 }
                 continue;

@@ -493,6 +493,29 @@ def test_flash_maxima_raised_block_after_block_into_a_strided_output(oracle, B, 
     status_ok()
 
 
+@pytest.mark.parametrize("B,N,H", [(37, 600, 4), (37, 513, 4), (20, 300, 16)])
+def test_flash_padding_warps_behind_a_working_item(oracle, B, N, H):
+    """CTAs that take several tile groups, where a group with rows for all warps is followed by one that leaves some warps (or a
+    whole tile) padding: those write the earlier item's rows while they only keep the later item's barriers moving. Whole groups
+    in equal rounds (444 groups, three a CTA, every third one padded) and the split form (640 groups), maxima raised on the way."""
+    from fastbb_b200 import _lib
+    from fastbb_b200.attention import attention
+    sms = torch.cuda.get_device_properties(dev()).multi_processor_count
+    groups = B * H * -(-N // 256)
+    if sms != 148:
+        pytest.skip("the shapes of this test are chosen for 148 SMs")
+    assert groups > sms and (groups % sms == 0) == (N != 300) and (_lib.load().fbb_flash64_workspace_bytes(B, N, H) > 0) == (N == 300)
+    g = torch.Generator().manual_seed(N)
+    q, k, v = (torch.randn(B, N, H, 64, generator=g).half() for _ in range(3))
+    q[:, ::3, :, 0] = 8.0  # as in the test above: some rows see a maximum that rises from block to block
+    k[..., 0] = (8.0 * (torch.arange(N) // 128)).half()[None, :, None]
+    out, check = padded((B, N, H, 64))
+    attention(q.to(dev()), k.to(dev()), v.to(dev()), out=out)
+    assert oracle.rel_l2(out.cpu().float(), oracle.attention(q, k, v)) < 2e-3
+    check()
+    status_ok()
+
+
 @pytest.mark.parametrize("variant", ["ff", "fh", "hh"])
 @pytest.mark.parametrize("N", [4097, 6145, 16385])
 def test_flash_full_size_properties(variant, N):
