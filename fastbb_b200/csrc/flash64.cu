@@ -581,7 +581,12 @@ flash64_umma_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
             const uint64_t vd = vd0 + (uint64_t)(s * (kTileBytes >> 4));
             umma_ts8_commit2_warp(dO, aP, vd, idesc_pv, first ? 0u : 1u, pv_done(t), v_empty(s));
             FBB_TRACE(2 + t, g, 2);
-            if (!have_next) break;
+            if (!have_next) {
+                // The CTA gives its tensor memory and barriers up when all warps are past their loops. A tile that ends in an item
+                // of padding has no softmax warp that waits for this last product, so the issuer does.
+                (void)all_ok(mbar_wait(pv_done(t), g & 1u, s_abort, DEV_TIMEOUT_TMEM_FULL, 10 + t));
+                break;
+            }
             it = nit;
             kb = nkb_;
             kb1 = nkb1;

@@ -516,6 +516,30 @@ def test_flash_padding_warps_behind_a_working_item(oracle, B, N, H):
     status_ok()
 
 
+@pytest.mark.parametrize("B,N,H", [(32, 257, 16), (1, 257, 80), (40, 128, 5)])
+def test_flash_last_item_with_a_tile_of_padding(oracle, B, N, H):
+    """CTAs whose last (or only) item leaves the second tile without a row: nobody reads that tile's last product, and the CTA
+    must still not leave before it is complete. Launches in turn with GEMMs, which take over the tensor memory at once."""
+    from fastbb_b200.attention import attention
+    from fastbb_b200.gemm import linear
+    g = torch.Generator().manual_seed(N + H)
+    qkv = torch.randn(B, N, 3, H, 64, generator=g).half()
+    w = (torch.randn(256, 64 * H, generator=g) / (64 * H) ** 0.5).half().to(dev())
+    qd, kd, vd = qkv.to(dev()).unbind(2)
+    first = None
+    for _ in range(20):
+        o = attention(qd, kd, vd, scale=0.125)
+        y = linear(o.view(B, N, H * 64), w)
+        first = (o, y) if first is None else first
+        assert torch.equal(o, first[0]) and torch.equal(y, first[1])
+    q, k, v = qkv.unbind(2)
+    b = [0, B // 2, B - 1]
+    want = oracle.attention(q[b], k[b], v[b], scale=0.125)
+    assert oracle.rel_l2(first[0][b].cpu().float(), want) < TOL_F32
+    assert oracle.rel_l2(first[1][b].cpu().float(), oracle.linear(first[0][b].cpu().reshape(3, N, H * 64), w.cpu())) < TOL_F32
+    status_ok()
+
+
 @pytest.mark.parametrize("variant", ["ff", "fh", "hh"])
 @pytest.mark.parametrize("N", [4097, 6145, 16385])
 def test_flash_full_size_properties(variant, N):
