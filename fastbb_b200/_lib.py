@@ -55,6 +55,7 @@ PROTOTYPES = {
     "fbb_diag_wait_timeout": (_i32, [ctypes.c_uint64, ctypes.c_uint, _vp]),
     "fbb_diag_sm_clock_mhz": (_i32, [_vp, _i64, _vp]),
     "fbb_linear_max_cta_pairs": (_i32, [_i32]),
+    "fbb_linear_form": (_i32, [_i64, _i32, _i32, _i32, _i32, ctypes.c_char_p, _i32]),
     "fbb_layernorm_f16": (_i32, [_vp, _vp, _vp, _vp, _i64, _i32, _i64, _i64, _f32, _i32, _i32, _vp]),
     "fbb_layernorm_split_f16": (_i32, [_vp, _vp, _vp, _vp, _vp, _vp, _i32, _i32, _i32, _i32, _f32, _i32, _i32, _vp]),
     "fbb_linear_f16": (_i32, [_vp, _vp, _vp, _vp, _vp, _vp, _i64, _i32, _i32, _i64, _i64, _i64, _i64, _i32, _i32, _vp]),

@@ -201,6 +201,14 @@ int fbb_linear_max_cta_pairs(int tile_columns) {
     return linear_max_pairs(tile_columns);
 }
 
+int fbb_linear_form(int64_t M, int N, int K, int epilogue, int out_overlaps_a, char* name, int name_bytes) {
+    if (name == nullptr) return fail(FBB_ERR_NULL, "linear_form: name is null");
+    if (epilogue < FBB_EPI_NONE || epilogue > FBB_EPI_SWIGLU) return fail(FBB_ERR_ENUM, "linear_form: unknown epilogue %d", epilogue);
+    if (M <= 0 || M > 0x7FFFFF00ll || N <= 0 || K <= 0 || (K & 7) != 0 || (N & 7) != 0 || name_bytes <= 0)
+        return fail(FBB_ERR_SHAPE, "linear_form: bad M/N/K (%lld, %d, %d) or name_bytes", (long long)M, N, K);
+    return linear_form(M, N, K, epilogue, out_overlaps_a != 0, name, name_bytes);
+}
+
 int fbb_layernorm_f16(const void* x, void* y, const void* w, const void* b, int64_t M, int C, int64_t ldx, int64_t ldy,
                       float eps, int in_dtype, int param_dtype, void* stream) {
     if (x == nullptr || y == nullptr) return fail(FBB_ERR_NULL, "layernorm: x or y is null");

@@ -21,6 +21,7 @@
 // In the persistent forms two accumulators (2 x BN columns) let the epilogue of tile i overlap the main loop of tile i+1;
 // the plain 256-column form cuts the tiles of a partly filled second wave into 128- or 64-column slices (narrow_tail).
 #include "common.cuh"
+#include <cstdio>
 #include <cstdlib>
 #include <mutex>
 
@@ -1487,6 +1488,142 @@ static bool gemm_pairs_enabled() {
 
 int linear_max_pairs(int bn) { return bn == 128 ? max_pairs<128, false>() : max_pairs<256, false>(); }
 
+// The form that a launch takes.
+struct LinearForm {
+    bool use_pairs = false, use128 = false;  // persistent form: CTA pairs; 128-column tiles
+    int wide_w = 0;                          // > 0: the wide pair form with items of this many columns
+    int split_bn = 0, split_s = 0;           // > 0: the split form with tiles of split_bn columns shared by split_s CTAs
+};
+
+// over_a: the output overlaps the A operand.
+static LinearForm choose_form(int64_t M, int N, int K, bool swiglu, bool over_a) {
+    const int n_out = swiglu ? N / 2 : N;
+    // Shape of the work item: one CTA with a 128x256 or 128x128 tile, or a CTA pair with a 256x256 tile (each CTA stages
+    // its 128 rows of A and half of the W rows, which cuts the operand traffic from L2 per FLOP by a third).
+    // Picked by a small cost model in units of one 128x256 one-CTA tile: waves of tiles over the workers (148 CTAs or 74
+    // pairs) times the relative tile time, fitted to measurements on B200: 128-column tiles 0.60 (they move 1.3x the
+    // operand bytes per FLOP), a pair's tile 0.895 per CTA plus a start-up term for the cluster launch that matters when
+    // the per-tile K loop is short (M = 32768, N = 4096, K = 1024: 219 us one-CTA, 196 us pairs; M = 6145: 48 vs 50 us).
+    // Pairs with 128-column tiles measured no better than single CTAs and are only reachable through the override.
+    // FBB_GEMM_FORCE = s256 | s128 | p256 | p128 | w<columns> | wa (the wide form's own width) | k<CTAs>x<columns> (the split
+    // form, where it takes the shape) overrides the choice (tuning aid).
+    const int sms = num_sms();
+    const bool pairs_ok = gemm_pairs_enabled();
+    const int pairs256 = pairs_ok ? (swiglu ? max_pairs<256, true>() : max_pairs<256, false>()) : 0;
+    auto waves = [](int64_t tiles, int workers) { return (double)((tiles + workers - 1) / workers); };
+    const int64_t tn256 = (n_out + 255) / 256, tn128 = (n_out + 127) / 128;
+    const int64_t dots = swiglu ? 2 * n_out : n_out;
+    // row tiles of a form: a remainder of a few rows gets none where launch_variant will leave it to the epilogue warps
+    // (a SwiGLU tile of 256 weight rows yields 128 output columns)
+    auto row_tiles_of = [&](int tile_rows, int64_t tiles_n, int workers, int bn) {
+        const int64_t tn = swiglu ? tn128 : tiles_n;
+        return remainder_by_gemv(M, tile_rows, tn, workers, dots, (int)K, bn) ? M / tile_rows : (M + tile_rows - 1) / tile_rows;
+    };
+    double best;
+    {
+        const int64_t t256 = row_tiles_of(BM, tn256, sms, 256) * tn256;
+        double tail = 0.0;
+        best = (!swiglu && narrow_tail(t256, sms, &tail) > 0) ? (double)(t256 / sms) + tail : waves(t256, sms) * 1.0;
+    }
+    bool use_pairs = false, use128 = false;
+    if (!swiglu) {
+        const double c = waves(row_tiles_of(BM, tn128, sms, 128) * tn128, sms) * 0.60;
+        if (n_out <= 128 || c < best) { best = c; use128 = true; }
+    }
+    if (pairs256 > 0) {
+        const double c = waves(row_tiles_of(2 * BM, tn256, pairs256, 256) * tn256, pairs256) * 0.895 + (K < 1536 ? 0.7 : 0.2);
+        if (c < best) { best = c; use_pairs = true; use128 = false; }
+    }
+    // The wide pair form (items of w <= 512 columns, one wave): a candidate when every item fits on the device at once with
+    // the narrowest such w and at least half of the pairs get an item. Its cost in the same units: 1.08 per 256 columns
+    // (its epilogue overlaps nothing) plus about 1.8 us of start-up, a unit being one 256-column tile's main loop
+    // (0.37 us per k-block + 1 us). Measured on B200 (us, wide against the best tiled form): M = 6145, N = 1024: K = 4096
+    // 39.6 / 46.0, K = 1024 15.4 / 17.5 (w = 352); M = 4097, N = 768, K = 3072 17.5 / 21.0 (w = 192); not taken where it
+    // measured slower: M = 5480, N = 1536 (w = 512: 25.6 / 22.8), M = 257 (a handful of items), and every shape with
+    // more than one wave of items (N = 4096: 68 / 48).
+    int wide_w = 0;  // > 0: the wide pair form with items of this many columns
+    const int wide_pairs = (pairs_ok && !swiglu) ? wide_max_pairs() : 0;
+    int wide_rule_w = 0;
+    if (wide_pairs > 0) {
+        const int64_t tmw = wide_row_tiles(M);
+        const int64_t max_chunks = tmw > 0 ? wide_pairs / tmw : 0;
+        if (max_chunks >= 1) {
+            int w = (int)(((n_out + max_chunks - 1) / max_chunks + 31) / 32 * 32);
+            if (w < 64) w = 64;
+            if (w <= kWideMaxCols && tmw * ((n_out + w - 1) / w) <= wide_pairs) wide_rule_w = w;
+        }
+        if (wide_rule_w > 0) {
+            const int64_t items = tmw * ((n_out + wide_rule_w - 1) / wide_rule_w);
+            const double unit_us = 0.37 * (double)((K + BK - 1) / BK) + 1.0;
+            const double c = (double)wide_rule_w / 256.0 * 1.08 + 1.8 / unit_us;
+            if (2 * items >= wide_pairs && c < best) wide_w = wide_rule_w;
+        }
+    }
+    // The split form: a candidate where its tiles times its cluster size fit the SMs at once, taken where its time (see
+    // split_cost_us) is below that of the forms above, 2.7 us and 0.9 of the model's units of time. Measured on B200 (us,
+    // without / with): M = 257: N = 384, K = 1536 8.4 / 4.8 (two CTAs per tile of 32 columns), K = 384 5.2 / 3.2 (one);
+    // N = 1152, K = 384 4.4 / 3.2; N = 768, K = 3072 13.2 / 7.5; N = 1024, K = 4096 16.3 / 9.6; M = 1041: N = 768, K = 3072
+    // 14.3 / 10.2, K = 768 6.5 / 4.9; M = 2056, N = 384, K = 1536 10.3 / 7.5.
+    // Not where the output overlaps A: a row's columns are then several CTAs' tiles, and one may write what another has still to
+    // read. (The persistent forms give up to 128 columns to one CTA, which has read its rows of A before it writes them.)
+    int split_bn = 0, split_s = 0;
+    if (!swiglu && !over_a && ((M + BM - 1) / BM) * tn128 <= sms) {  // (its widest tiles, one CTA each, fit the SMs at once)
+        const SplitClusters& most = split_max_clusters();
+        const double unit_us = 0.37 * (double)((K + BK - 1) / BK) + 1.0;
+        double split_best = 2.7 + 0.9 * unit_us * best;
+        if (wide_w > 0) {  // a k-block of a wide item takes no less than 0.2 us, and its epilogue overlaps nothing
+            const double kb_us = 0.44 * (double)wide_w / 352.0;
+            split_best = 2.7 + 0.02 * (double)wide_w + (double)((K + BK - 1) / BK) * (kb_us > 0.2 ? kb_us : 0.2);
+        }
+        for (int ks = 1; ks <= 8; ks *= 2) {
+            for (int bn = 32; bn <= 128; bn *= 2) {
+                if (!split_fits(most, M, N, K, bn, ks) || split_cost_us(K, bn, ks) >= split_best) continue;
+                split_best = split_cost_us(K, bn, ks);
+                split_bn = bn;
+                split_s = ks;
+            }
+        }
+    }
+    if (const char* f = getenv("FBB_GEMM_FORCE")) {
+        wide_w = 0;
+        split_bn = 0;
+        if (f[0] == 'k' && !swiglu && !over_a) {
+            char* end = nullptr;
+            const int ks = (int)strtol(f + 1, &end, 10), bn = *end == 'x' ? atoi(end + 1) : 0;
+            if (split_fits(split_max_clusters(), M, N, K, bn, ks)) {
+                split_bn = bn;
+                split_s = ks;
+            }
+        }
+        if (f[0] == 'w' && !swiglu && wide_max_pairs() > 0) {
+            const int w = f[1] == 'a' ? wide_rule_w : atoi(f + 1);  // "wa": the rule's own width, whatever the cost model says
+            if (w >= 32 && w <= kWideMaxCols && (w & 31) == 0) wide_w = w;
+        }
+        const bool want128 = f[0] != '\0' && f[1] == '1' && !swiglu;  // SwiGLU always uses 256-column tiles (x1 | x2 halves)
+        if (f[0] == 's' || (f[0] == 'p' && pairs256 > 0 && (!want128 || max_pairs<128, false>() > 0))) {
+            use_pairs = f[0] == 'p';
+            use128 = want128;
+        }
+    }
+
+    LinearForm form;
+    form.use_pairs = use_pairs;
+    form.use128 = use128;
+    form.wide_w = wide_w;
+    form.split_bn = split_bn;
+    form.split_s = split_s;
+    return form;
+}
+
+int linear_form(int64_t M, int N, int K, int epilogue, bool over_a, char* name, int bytes) {
+    const LinearForm f = choose_form(M, N, K, epilogue == FBB_EPI_SWIGLU, over_a);
+    int n;
+    if (f.split_bn > 0) n = snprintf(name, (size_t)bytes, "k%dx%d", f.split_s, f.split_bn);
+    else if (f.wide_w > 0) n = snprintf(name, (size_t)bytes, "w%d", f.wide_w);
+    else n = snprintf(name, (size_t)bytes, "%c%d", f.use_pairs ? 'p' : 's', f.use128 ? 128 : 256);
+    return n < bytes ? FBB_OK : fail(FBB_ERR_SHAPE, "linear_form: the name needs %d bytes", n + 1);
+}
+
 int launch_linear(const void* A, const void* W, void* C, const void* bias, const void* res, const void* gamma, int64_t M,
                   int N, int K, int64_t lda, int64_t ldw, int64_t ldc, int64_t ldr, int epilogue, int accumulate,
                   cudaStream_t stream, bool w_early) {
@@ -1513,113 +1650,12 @@ int launch_linear(const void* A, const void* W, void* C, const void* bias, const
     g.gemv_row0 = (int)M;
     g.gemv_rows = 0;
 
-    // Shape of the work item: one CTA with a 128x256 or 128x128 tile, or a CTA pair with a 256x256 tile (each CTA stages
-    // its 128 rows of A and half of the W rows, which cuts the operand traffic from L2 per FLOP by a third).
-    // Picked by a small cost model in units of one 128x256 one-CTA tile: waves of tiles over the workers (148 CTAs or 74
-    // pairs) times the relative tile time, fitted to measurements on B200: 128-column tiles 0.60 (they move 1.3x the
-    // operand bytes per FLOP), a pair's tile 0.895 per CTA plus a start-up term for the cluster launch that matters when
-    // the per-tile K loop is short (M = 32768, N = 4096, K = 1024: 219 us one-CTA, 196 us pairs; M = 6145: 48 vs 50 us).
-    // Pairs with 128-column tiles measured no better than single CTAs and are only reachable through the override.
-    // FBB_GEMM_FORCE = s256 | s128 | p256 | p128 | w<columns> | wa (the wide form's own width) overrides the choice (tuning aid).
-    const int sms = num_sms();
-    const bool pairs_ok = gemm_pairs_enabled();
-    const int pairs256 = pairs_ok ? (swiglu ? max_pairs<256, true>() : max_pairs<256, false>()) : 0;
-    auto waves = [](int64_t tiles, int workers) { return (double)((tiles + workers - 1) / workers); };
-    const int64_t tn256 = (g.n_out + 255) / 256, tn128 = (g.n_out + 127) / 128;
-    const int64_t dots = swiglu ? 2 * g.n_out : g.n_out;
-    // row tiles of a form: a remainder of a few rows gets none where launch_variant will leave it to the epilogue warps
-    // (a SwiGLU tile of 256 weight rows yields 128 output columns)
-    auto row_tiles_of = [&](int tile_rows, int64_t tiles_n, int workers, int bn) {
-        const int64_t tn = swiglu ? tn128 : tiles_n;
-        return remainder_by_gemv(M, tile_rows, tn, workers, dots, (int)K, bn) ? M / tile_rows : (M + tile_rows - 1) / tile_rows;
-    };
-    double best;
-    {
-        const int64_t t256 = row_tiles_of(BM, tn256, sms, 256) * tn256;
-        double tail = 0.0;
-        best = (!swiglu && narrow_tail(t256, sms, &tail) > 0) ? (double)(t256 / sms) + tail : waves(t256, sms) * 1.0;
-    }
-    bool use_pairs = false, use128 = false;
-    if (!swiglu) {
-        const double c = waves(row_tiles_of(BM, tn128, sms, 128) * tn128, sms) * 0.60;
-        if (g.n_out <= 128 || c < best) { best = c; use128 = true; }
-    }
-    if (pairs256 > 0) {
-        const double c = waves(row_tiles_of(2 * BM, tn256, pairs256, 256) * tn256, pairs256) * 0.895 + (K < 1536 ? 0.7 : 0.2);
-        if (c < best) { best = c; use_pairs = true; use128 = false; }
-    }
-    // The wide pair form (items of w <= 512 columns, one wave): a candidate when every item fits on the device at once with
-    // the narrowest such w and at least half of the pairs get an item. Its cost in the same units: 1.08 per 256 columns
-    // (its epilogue overlaps nothing) plus about 1.8 us of start-up, a unit being one 256-column tile's main loop
-    // (0.37 us per k-block + 1 us). Measured on B200 (us, wide against the best tiled form): M = 6145, N = 1024: K = 4096
-    // 39.6 / 46.0, K = 1024 15.4 / 17.5 (w = 352); M = 4097, N = 768, K = 3072 17.5 / 21.0 (w = 192); not taken where it
-    // measured slower: M = 5480, N = 1536 (w = 512: 25.6 / 22.8), M = 257 (a handful of items), and every shape with
-    // more than one wave of items (N = 4096: 68 / 48).
-    int wide_w = 0;  // > 0: the wide pair form with items of this many columns
-    const int wide_pairs = (pairs_ok && !swiglu) ? wide_max_pairs() : 0;
-    int wide_rule_w = 0;
-    if (wide_pairs > 0) {
-        const int64_t tmw = wide_row_tiles(M);
-        const int64_t max_chunks = tmw > 0 ? wide_pairs / tmw : 0;
-        if (max_chunks >= 1) {
-            int w = (int)(((g.n_out + max_chunks - 1) / max_chunks + 31) / 32 * 32);
-            if (w < 64) w = 64;
-            if (w <= kWideMaxCols && tmw * ((g.n_out + w - 1) / w) <= wide_pairs) wide_rule_w = w;
-        }
-        if (wide_rule_w > 0) {
-            const int64_t items = tmw * ((g.n_out + wide_rule_w - 1) / wide_rule_w);
-            const double unit_us = 0.37 * (double)((K + BK - 1) / BK) + 1.0;
-            const double c = (double)wide_rule_w / 256.0 * 1.08 + 1.8 / unit_us;
-            if (2 * items >= wide_pairs && c < best) wide_w = wide_rule_w;
-        }
-    }
-    // The split form: a candidate where its tiles times its cluster size fit the SMs at once, taken where its time (see
-    // split_cost_us) is below that of the forms above, 2.7 us and 0.9 of the model's units of time. Measured on B200 (us,
-    // without / with): M = 257: N = 384, K = 1536 8.4 / 4.8 (two CTAs per tile of 32 columns), K = 384 5.2 / 3.2 (one);
-    // N = 1152, K = 384 4.4 / 3.2; N = 768, K = 3072 13.2 / 7.5; N = 1024, K = 4096 16.3 / 9.6; M = 1041: N = 768, K = 3072
-    // 14.3 / 10.2, K = 768 6.5 / 4.9; M = 2056, N = 384, K = 1536 10.3 / 7.5.
-    int split_bn = 0, split_s = 0;
-    if (!swiglu && ((M + BM - 1) / BM) * tn128 <= sms) {  // (its widest tiles, one CTA each, fit the SMs at once)
-        const SplitClusters& most = split_max_clusters();
-        const double unit_us = 0.37 * (double)((K + BK - 1) / BK) + 1.0;
-        double split_best = 2.7 + 0.9 * unit_us * best;
-        if (wide_w > 0) {  // a k-block of a wide item takes no less than 0.2 us, and its epilogue overlaps nothing
-            const double kb_us = 0.44 * (double)wide_w / 352.0;
-            split_best = 2.7 + 0.02 * (double)wide_w + (double)((K + BK - 1) / BK) * (kb_us > 0.2 ? kb_us : 0.2);
-        }
-        for (int ks = 1; ks <= 8; ks *= 2) {
-            for (int bn = 32; bn <= 128; bn *= 2) {
-                if (!split_fits(most, M, N, K, bn, ks) || split_cost_us(K, bn, ks) >= split_best) continue;
-                split_best = split_cost_us(K, bn, ks);
-                split_bn = bn;
-                split_s = ks;
-            }
-        }
-    }
-    if (const char* f = getenv("FBB_GEMM_FORCE")) {
-        wide_w = 0;
-        split_bn = 0;
-        if (f[0] == 'k' && !swiglu) {
-            char* end = nullptr;
-            const int ks = (int)strtol(f + 1, &end, 10), bn = *end == 'x' ? atoi(end + 1) : 0;
-            if (split_fits(split_max_clusters(), M, N, K, bn, ks)) {
-                split_bn = bn;
-                split_s = ks;
-            }
-        }
-        if (f[0] == 'w' && !swiglu && wide_max_pairs() > 0) {
-            const int w = f[1] == 'a' ? wide_rule_w : atoi(f + 1);  // "wa": the rule's own width, whatever the cost model says
-            if (w >= 32 && w <= kWideMaxCols && (w & 31) == 0) wide_w = w;
-        }
-        const bool want128 = f[0] != '\0' && f[1] == '1' && !swiglu;  // SwiGLU always uses 256-column tiles (x1 | x2 halves)
-        if (f[0] == 's' || (f[0] == 'p' && pairs256 > 0 && (!want128 || max_pairs<128, false>() > 0))) {
-            use_pairs = f[0] == 'p';
-            use128 = want128;
-        }
-    }
-
-    if (split_bn > 0) return launch_split(A, W, g, lda, ldw, split_bn, split_s, w_early, stream);
-    if (wide_w > 0) return launch_wide(A, W, C, g, lda, ldw, wide_w, stream);
+    const uintptr_t a0 = reinterpret_cast<uintptr_t>(A), c0 = reinterpret_cast<uintptr_t>(C);
+    const bool over_a = a0 < c0 + 2 * (uintptr_t)((M - 1) * ldc + g.n_out) && c0 < a0 + 2 * (uintptr_t)((M - 1) * lda + K);
+    const LinearForm form = choose_form(M, N, K, swiglu, over_a);
+    if (form.split_bn > 0) return launch_split(A, W, g, lda, ldw, form.split_bn, form.split_s, w_early, stream);
+    if (form.wide_w > 0) return launch_wide(A, W, C, g, lda, ldw, form.wide_w, stream);
+    const bool use_pairs = form.use_pairs, use128 = form.use128;
 
     CUtensorMap ta, tw;
     uint64_t dims_a[2] = {(uint64_t)K, (uint64_t)M};

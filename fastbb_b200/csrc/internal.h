@@ -76,6 +76,9 @@ int launch_linear(const void* A, const void* W, void* C, const void* bias, const
                   int N, int K, int64_t lda, int64_t ldw, int64_t ldc, int64_t ldr, int epilogue, int accumulate,
                   cudaStream_t stream, bool w_early = false);
 
+// Name of the form such a launch takes, as FBB_GEMM_FORCE spells it, without launching anything. over_a: C overlaps A.
+int linear_form(int64_t M, int N, int K, int epilogue, bool over_a, char* name, int bytes);
+
 // The same followed by y = LayerNorm(C) * ln_w + ln_b (rows of N elements), fused into the GEMM launch when the shape
 // allows. `counter`: 4 bytes of zeroed device memory that every launch leaves zero (needed when M has remainder rows).
 int launch_linear_layernorm(const void* A, const void* W, void* C, const void* bias, const void* res, const void* gamma, int64_t M, int N,

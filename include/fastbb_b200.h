@@ -92,6 +92,11 @@ int fbb_diag_sm_clock_mhz(float* out_mhz, int64_t spin_clocks, void* stream);
  * once; 0 means the kernel runs in its one-CTA form. No counterpart in the reference (its GEMMs are cuBLAS calls). */
 int fbb_linear_max_cta_pairs(int tile_columns);
 
+/* Diagnostics: the form that fbb_linear_f16 takes for these sizes on the current device, spelled as in FBB_GEMM_FORCE ("s128",
+ * "p256", "w352", "k2x32", ...), written to name (16 bytes hold every one). out_overlaps_a != 0: C shares memory with A. No
+ * counterpart in the reference. */
+int fbb_linear_form(int64_t M, int N, int K, int epilogue, int out_overlaps_a, char* name, int name_bytes);
+
 /* y[m, :] = LayerNorm(x[m, :]) * w + b, statistics in fp32, output fp16.
  * Replaces: the nn.LayerNorm calls of fastbb/vit.py:114,126,130,139,159,166,170 (norm1 / norm2) and :184,241 (vit.norm).
  * x: [M, C] of in_dtype with row stride ldx; y: [M, C] fp16 with row stride ldy; w, b: [C] of param_dtype or null.

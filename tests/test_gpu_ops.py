@@ -218,6 +218,32 @@ def test_linear_split_form_matches_oracle(oracle, ctas, bn, monkeypatch):
     status_ok()
 
 
+def linear_form(M, N, K, epilogue=0, over_a=0):
+    """The form a linear() launch takes, spelled as in FBB_GEMM_FORCE."""
+    import ctypes
+    from fastbb_b200 import _lib
+    name = ctypes.create_string_buffer(16)
+    _lib.check(_lib.load().fbb_linear_form(M, N, K, epilogue, over_a, name, len(name)))
+    return name.value.decode()
+
+
+@pytest.mark.parametrize("M", [1, 128, 129, 1024])
+@pytest.mark.parametrize("N,shared", [(128, False), (72, False), (128, True)])
+def test_linear_in_place_on_its_input(oracle, M, N, shared):
+    """out is x (N = K <= 128), alone or as residual too: one CTA must own all columns of a row, or another may read what it wrote."""
+    from fastbb_b200.gemm import linear
+    assert linear_form(M, N, N, 0, 1) == "s128"
+    g = torch.Generator().manual_seed(M + N)
+    x = torch.randn(M, N, generator=g).half()
+    w = (torch.randn(N, N, generator=g) / N ** 0.5).half()
+    want = oracle.linear(x, w, None, res=x if shared else None)
+    for _ in range(20):
+        xd = x.to(dev())
+        y = linear(xd, w.to(dev()), None, res=xd if shared else None, variant="f32", out=xd)
+        assert y.data_ptr() == xd.data_ptr() and oracle.rel_l2(y.cpu().float(), want) < TOL_F32
+    status_ok()
+
+
 @pytest.mark.parametrize("M,N,K,act,variant", [(2561, 2000, 136, "gelu", "f32"), (2561, 1848, 72, None, "h"), (6145, 1024, 64, None, "f32"),
                                                 (2600, 2048, 200, None, "f32")])
 def test_linear_last_wave_in_slices_equals_whole_tiles(oracle, M, N, K, act, variant, monkeypatch):
