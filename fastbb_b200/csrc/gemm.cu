@@ -879,6 +879,7 @@ struct SplitArgs {
     int act, acc_f16;
     int bn, tiles_n;           // tile width (32, 64 or 128); tiles per row of tiles
     int stages, stage_bytes;   // operand ring: A tile (16 KB) | bn rows of W
+    int load_bytes;            // of a stage: what its two loads bring (fewer rows of A when M < 128)
     int w_early;               // W was complete before the previous launch started: load it ahead of the dependency wait
 };
 
@@ -926,7 +927,7 @@ linear_split_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
         fence_barrier_init();
         if (g.w_early) {
             for (int i = 0; i < g.stages && i < nkb; ++i) {
-                mbar_arrive_expect_tx(full_bar(i), (uint32_t)g.stage_bytes);
+                mbar_arrive_expect_tx(full_bar(i), (uint32_t)g.load_bytes);
                 tma_load_2d(base + i * g.stage_bytes + BM * BK * 2, &tmap_w, full_bar(i), (kb0 + i) * BK, n0);
             }
         }
@@ -964,7 +965,7 @@ linear_split_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
             if (__all_sync(0xffffffffu, ok) == 0) { ok = false; break; }
             const uint32_t sa = base + s * g.stage_bytes;
             if (g.w_early && i < g.stages) tma_load_2d_warp(sa, &tmap_a, full_bar(s), (kb0 + i) * BK, m0);
-            else tma_load_2d_two_warp(full_bar(s), (uint32_t)g.stage_bytes, sa, &tmap_a, (kb0 + i) * BK, m0, sa + BM * BK * 2, &tmap_w, (kb0 + i) * BK, n0);
+            else tma_load_2d_two_warp(full_bar(s), (uint32_t)g.load_bytes, sa, &tmap_a, (kb0 + i) * BK, m0, sa + BM * BK * 2, &tmap_w, (kb0 + i) * BK, n0);
             if (++s == g.stages) { s = 0; ph ^= 1u; }
         }
         if (!ok) __nanosleep(20000);  // let copies already in flight land before the CTA leaves
@@ -1145,12 +1146,17 @@ static int launch_split(const void* A, const void* W, const GemmArgs& base, int6
     CUtensorMap ta, tw;
     uint64_t dims_a[2] = {(uint64_t)g.K, (uint64_t)g.M};
     int64_t str_a[2] = {1, lda};
-    uint32_t box_a[2] = {BK, BM};
+    // A box of no more rows than there are, to the next eight: rows outside the tensor are not free to load, the less so the more
+    // CTAs load them. N = 3072, K = 768 (96 CTAs), us with boxes of 128 rows / of M rows, and the 128-column form: M = 17 6.6 / 4.2,
+    // 6.4; M = 33 6.2 / 4.3; M = 64 5.5 / 4.3; N = 2304, K = 768 (144 CTAs), M = 17: 5.5 / 3.8, 5.3. The rows of the tile that
+    // are not loaded hold anything, also NaN; they reach only output rows that do not exist.
+    uint32_t box_a[2] = {BK, g.M < BM ? (uint32_t)((g.M + 7) & ~7) : BM};
     int st = make_tmap_f16(&ta, A, 2, dims_a, str_a, box_a);
     if (st != FBB_OK) return st;
     uint64_t dims_w[2] = {(uint64_t)g.K, (uint64_t)g.N};
     int64_t str_w[2] = {1, ldw};
     uint32_t box_w[2] = {BK, (uint32_t)bn};
+    g.load_bytes = (int)(box_a[1] + box_w[1]) * BK * 2;
     st = make_tmap_f16(&tw, W, 2, dims_w, str_w, box_w);
     if (st != FBB_OK) return st;
     const unsigned grid = (unsigned)(((g.M + BM - 1) / BM) * g.tiles_n * s);

@@ -227,6 +227,25 @@ def linear_form(M, N, K, epilogue=0, over_a=0):
     return name.value.decode()
 
 
+@pytest.mark.parametrize("M", [1, 7, 8, 9, 33, 63, 64, 65, 120, 121, 127])
+def test_linear_split_form_of_fewer_rows_than_a_tile(oracle, M):
+    """A tile of the split form loads no more rows of x than there are (to the next eight). What the rest of its shared memory
+    holds - NaN here, from the launch before - must not reach a row of the output."""
+    from fastbb_b200.gemm import linear
+    g = torch.Generator().manual_seed(M)
+    for N, K, variant in [(2304, 768, "f32"), (384, 1536, "h"), (264, 328, "f32")]:
+        assert linear_form(M, N, K).startswith("k")
+        w = (torch.randn(N, K, generator=g) / K ** 0.5).half().to(dev())
+        x = torch.randn(M, K, generator=g).half()
+        res = torch.randn(M, N, generator=g).half()
+        assert linear(torch.full((128, K), float("nan"), dtype=torch.float16, device=dev()), w).isnan().all()
+        out, check = padded((M, N))
+        y = linear(x.to(dev()), w, None, res=res.to(dev()), variant=variant, out=out)
+        assert oracle.rel_l2(y.cpu().float(), oracle.linear(x, w.cpu(), None, res=res)) < (TOL_F16 if variant == "h" else TOL_F32), (N, K)
+        check()
+    status_ok()
+
+
 @pytest.mark.parametrize("M", [1, 128, 129, 1024])
 @pytest.mark.parametrize("N,shared", [(128, False), (72, False), (128, True)])
 def test_linear_in_place_on_its_input(oracle, M, N, shared):
