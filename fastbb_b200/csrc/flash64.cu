@@ -467,29 +467,22 @@ flash64_umma_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
         if (lane == 0) {
             int s = 0;
             uint32_t ph = 0;
-            // Q of an item goes to one of two buffers, so that the next item's is there when a tile gets to it: the tiles run
-            // about a unit and a half apart, and neither waits for the other at the end of an item.
-            auto load_q = [&](int it) -> bool {
-                int w, kb0, kb1;
-                item_at(it, w, kb0, kb1);
-                const int bh = w / a.groups_per_head;
-                const int q0 = (w - bh * a.groups_per_head) * (FQ * NQ);
-                const int b = bh / a.H, h = bh - b * a.H;
-                const int i = it & 1;
-                if (!mbar_wait(q_empty(i), (((uint32_t)it >> 1) & 1u) ^ 1u, s_abort, DEV_TIMEOUT_SMEM_EMPTY, 32)) return false;
-                mbar_arrive_expect_tx(q_full(i), NQ * kTileBytes);
-                for (int t = 0; t < NQ; ++t) tma_load_4d(base + S::kQOff + (2 * i + t) * kTileBytes, &tmap_q, q_full(i), 0, h, q0 + t * FQ, b);
-                return true;
-            };
-            bool ok = n_items == 0 || load_q(0);
+            bool ok = true;
 #pragma unroll 1
             for (int it = 0; it < n_items && ok; ++it) {
                 int w, kb0, kb1;
                 item_at(it, w, kb0, kb1);
                 const int bh = w / a.groups_per_head;
+                const int q0 = (w - bh * a.groups_per_head) * (FQ * NQ);
                 const int b = bh / a.H, h = bh - b * a.H;
-                // not before this item's first units: the other buffer is free once both tiles have left the previous item
-                const int kq = it + 1 < n_items ? min(kb0 + kKVStages, kb1 - 1) : -1;
+                // Q goes to one of two buffers, free when both tiles have left the item before the previous one. The tiles run about
+                // a unit and a half apart and up to four units behind this loop: the next Q is there when a tile gets to it.
+                // (One code path for all items: a separate load of the first Q put 1100 clocks between it and the first K, the
+                // coordinates worked out twice and instruction fetches in between, where 400 do.)
+                const int i = it & 1;
+                if (!mbar_wait(q_empty(i), (((uint32_t)it >> 1) & 1u) ^ 1u, s_abort, DEV_TIMEOUT_SMEM_EMPTY, 32)) { ok = false; break; }
+                mbar_arrive_expect_tx(q_full(i), NQ * kTileBytes);
+                for (int t = 0; t < NQ; ++t) tma_load_4d(base + S::kQOff + (2 * i + t) * kTileBytes, &tmap_q, q_full(i), 0, h, q0 + t * FQ, b);
 #pragma unroll 1
                 for (int kb = kb0; kb < kb1; ++kb) {
                     if (!mbar_wait(k_empty(s), ph ^ 1u, s_abort, DEV_TIMEOUT_SMEM_EMPTY, s)) { ok = false; break; }
@@ -499,7 +492,6 @@ flash64_umma_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
                     mbar_arrive_expect_tx(v_full(s), kTileBytes);
                     tma_load_4d(base + S::kVOff + s * kTileBytes, &tmap_v, v_full(s), 0, h, kb * FK, b);
                     if (++s == kKVStages) { s = 0; ph ^= 1u; }
-                    if (kb == kq && !load_q(it + 1)) { ok = false; break; }
                 }
             }
             if (!ok) __nanosleep(20000);
