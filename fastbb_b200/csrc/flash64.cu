@@ -31,8 +31,8 @@
 //                   the first blocks); otherwise P is taken relative to the older maximum, which keeps it <= 256 and
 //                   exactly as accurate in fp16. The loop over an item's blocks holds only what every block needs: each
 //                   thread compares its own share of a row with the row's limit and the warp votes (no shuffles), and a
-//                   block that has to raise the maximum, or is ragged, leaves for a second loop that reads S again from
-//                   tensor memory in halves. An item's first block (which takes the maximum) stands before the loop, its
+//                   block that has to raise the maximum leaves for code that reads S again from tensor memory in halves; a
+//                   ragged last block has a masking copy of the loop's code behind it. An item's first block (which takes the maximum) stands before the loop, its
 //                   rows are written by 16-row TMA stores in the NEXT item's first block, behind that block's
 //                   exponentials, and Q has two buffers, so that neither tile stops between items. With one loop for all
 //                   of this and the write-out between items: 1531 / 213.6 / 81.8 us at N = 16385 / 6145 / 4097 (16 / 16 /
@@ -62,6 +62,7 @@
 // then exponentials, then sums) compiles to the same schedule; writing P back in two halves costs a second wait (212 us).
 #include "common.cuh"
 #include <cstdlib>
+#include <type_traits>
 
 #include "internal.h"
 
@@ -681,10 +682,11 @@ flash64_umma_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
                             pack_h2(__uint_as_float(o[4 * k + 4]) * invA, __uint_as_float(o[4 * k + 5]) * invA),
                             pack_h2(__uint_as_float(o[4 * k + 6]) * invB, __uint_as_float(o[4 * k + 7]) * invB));
             }
+            const int row0 = (w - bh * a.groups_per_head) * (FQ * NQ) + t * FQ + lane_base;
             fence_proxy_async_smem();
             __syncwarp();
             if (lane == 0) {
-                tma_store_4d(&tmap_o, st, 0, h, (w - bh * a.groups_per_head) * (FQ * NQ) + t * FQ + lane_base, b);
+                tma_store_4d(&tmap_o, st, 0, h, row0, b);
                 bulk_commit();
             }
             return true;
@@ -728,12 +730,25 @@ flash64_umma_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
             }
             const bool ragged = to_end && (a.N & (FK - 1)) != 0;  // the group's last key block has keys beyond N
             const int key0 = (nkb - 1) * FK + 2 * cq;
+            // That block has no key in its upper half. A ragged block goes through S once like any other, with its own copy of the
+            // code (masks, half of the work where half is empty). Through the two passes of the blocks that raise a maximum, us
+            // with / now: 1 x 223 tokens x 16 heads 6.26 / 5.74, 32 x 257 x 16 56.5 / 53.2, 4 x 1370 x 12 39.8 / 38.0.
+            const bool half = a.N - (nkb - 1) * FK <= 64;
             {
                 // ---- the item's first unit takes the running maxima
                 if (!mbar_wait(s_full(t), g & 1u, s_abort, DEV_TIMEOUT_TMEM_FULL, t)) { ok = false; break; }
                 tc_fence_after();
                 uint32_t sc[64], pk[32];
-                tmem_ld_16x256b_x16(tS, sc);
+                float mxA, mxB;
+                // In halves in the one-tile kernel, whose launches are the short ones: the upper half of a ragged block may hold no
+                // key. (The two-tile kernel has no registers to spare for this.)
+                const bool lower = NQ == 1 && half && ragged && n == 1;
+                if constexpr (NQ == 1) {
+                    tmem_ld_16x256b_x8(tS, sc);
+                    if (!lower) tmem_ld_16x256b_x8(tS + 64u, sc + 32);
+                } else {
+                    tmem_ld_16x256b_x16(tS, sc);
+                }
                 tmem_wait_ld();
                 tmem_tie32(sc);
                 tmem_tie32(sc + 32);
@@ -741,11 +756,20 @@ flash64_umma_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
                 __syncwarp();
                 if (lane == 0) mbar_arrive(s_free(t));
                 if (ragged && n == 1) {
-                    mask_frag(sc, key0, a.N);
-                    mask_frag(sc + 32, key0 + 64, a.N);
+                    if (half || NQ == 2) mask_frag(sc, key0, a.N);
+                    if (!half || NQ == 2) mask_frag(sc + 32, key0 + 64, a.N);
                 }
-                float mxA, mxB;
-                max_frag<16>(sc, mxA, mxB);
+                if constexpr (NQ == 1) {
+                    max_frag<8>(sc, mxA, mxB);
+                    if (!lower) {
+                        float xA, xB;
+                        max_frag<8>(sc + 32, xA, xB);
+                        mxA = fmaxf(mxA, xA);
+                        mxB = fmaxf(mxB, xB);
+                    }
+                } else {
+                    max_frag<16>(sc, mxA, mxB);
+                }
                 mxA = fmaxf(mxA, __shfl_xor_sync(0xffffffffu, mxA, 1));
                 mxB = fmaxf(mxB, __shfl_xor_sync(0xffffffffu, mxB, 1));
                 mxA = fmaxf(mxA, __shfl_xor_sync(0xffffffffu, mxA, 2));
@@ -755,7 +779,17 @@ flash64_umma_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
                 tA = mxA + lazy;
                 tB = mxB + lazy;
                 float2 accA = make_float2(0.f, 0.f), accB = make_float2(0.f, 0.f);
-                exp_frag<16>(sc, sl, mA, mB, accA, accB, pk);
+                if constexpr (NQ == 1) {
+                    exp_frag<8>(sc, sl, mA, mB, accA, accB, pk);
+                    if (!lower) {
+                        exp_frag<8>(sc + 32, sl, mA, mB, accA, accB, pk + 16);
+                    } else {
+#pragma unroll
+                        for (int i = 16; i < 32; ++i) pk[i] = 0u;
+                    }
+                } else {
+                    exp_frag<16>(sc, sl, mA, mB, accA, accB, pk);
+                }
                 if (g > 0) {
                     if (!mbar_wait(pv_done(t), (g - 1u) & 1u, s_abort, DEV_TIMEOUT_TMEM_FULL, 8 + t)) { ok = false; break; }
                     tc_fence_after();
@@ -772,50 +806,85 @@ flash64_umma_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
                 ++g;
             }
             int plain = n - (ragged ? 1 : 0);
-#pragma unroll 1
-            while (n > 0) {
-                // ---- the units that are all alike
+            // One unit in a single pass over S, in registers: kDone, kRaise (a row's maximum must be raised first; nothing has been
+            // released or written) or kFail (a wait ran out).
+            enum { kDone, kRaise, kFail };
+            auto unit = [&](auto masked) -> int {
+                FBB_TRACE(4 + u + 8 * t, g, 0);
+                if (!mbar_wait(s_full(t), g & 1u, s_abort, DEV_TIMEOUT_TMEM_FULL, t)) return kFail;
+                tc_fence_after();
+                FBB_TRACE(4 + u + 8 * t, g, 1);
+                uint32_t sc[64], pk[32];
+                float mxA, mxB;
                 float2 accA = make_float2(0.f, 0.f), accB = make_float2(0.f, 0.f);
-#pragma unroll 1
-                for (; plain > 0; --plain, --n, ++g) {
-                    FBB_TRACE(4 + u + 8 * t, g, 0);
-                    if (!mbar_wait(s_full(t), g & 1u, s_abort, DEV_TIMEOUT_TMEM_FULL, t)) { ok = false; break; }
-                    tc_fence_after();
-                    FBB_TRACE(4 + u + 8 * t, g, 1);
-                    uint32_t sc[64], pk[32];
+                if constexpr (decltype(masked)::value) {
+                    if (half) {  // no key in the block's upper half
+                        tmem_ld_16x256b_x8(tS, sc);
+                        tmem_wait_ld();
+                        tmem_tie32(sc);
+                        mask_frag(sc, key0, a.N);
+                        max_frag<8>(sc, mxA, mxB);
+                        if (__any_sync(0xffffffffu, mxA > tA || mxB > tB)) return kRaise;
+                        tc_fence_before();
+                        __syncwarp();
+                        if (lane == 0) mbar_arrive(s_free(t));
+                        exp_frag<8>(sc, sl, mA, mB, accA, accB, pk);
+#pragma unroll
+                        for (int i = 16; i < 32; ++i) pk[i] = 0u;
+                    }
+                }
+                if (!decltype(masked)::value || !half) {
                     tmem_ld_16x256b_x16(tS, sc);
                     tmem_wait_ld();
                     tmem_tie32(sc);
                     tmem_tie32(sc + 32);
-                    float mxA, mxB;
+                    if constexpr (decltype(masked)::value) mask_frag(sc + 32, key0 + 64, a.N);
                     max_frag<16>(sc, mxA, mxB);
-                    accA = make_float2(0.f, 0.f);
-                    accB = make_float2(0.f, 0.f);
                     exp_frag<kEarly>(sc, sl, mA, mB, accA, accB, pk);
-                    if (__any_sync(0xffffffffu, mxA > tA || mxB > tB)) break;
+                    if (__any_sync(0xffffffffu, mxA > tA || mxB > tB)) return kRaise;
                     tc_fence_before();
                     __syncwarp();
                     if (lane == 0) mbar_arrive(s_free(t));  // S_t is in registers: the next Q K^T may overwrite it
                     FBB_TRACE(4 + u + 8 * t, g, 2);
                     exp_frag<16 - kEarly>(sc + 4 * kEarly, sl, mA, mB, accA, accB, pk + 2 * kEarly);
-                    // P_t is read by the previous unit's P.V until that product has completed: waiting here, not before the
-                    // exponentials, keeps the issue and run time of that product off the softmax warps' path
-                    if (!mbar_wait(pv_done(t), (g - 1u) & 1u, s_abort, DEV_TIMEOUT_TMEM_FULL, 8 + t)) { ok = false; break; }
-                    tc_fence_after();
-                    tmem_st_16x128b_x16(tO + kColP, pk);
-                    FBB_TRACE(4 + u + 8 * t, g, 3);
-                    tmem_wait_st();
-                    tc_fence_before();
-                    __syncwarp();
-                    if (lane == 0) mbar_arrive(p_ready(t));
-                    FBB_TRACE(4 + u + 8 * t, g, 4);
-                    lA += accA.x + accA.y;
-                    lB += accB.x + accB.y;
                 }
+                // P_t is read by the previous unit's P.V until that product has completed: waiting here, not before the
+                // exponentials, keeps the issue and run time of that product off the softmax warps' path
+                if (!mbar_wait(pv_done(t), (g - 1u) & 1u, s_abort, DEV_TIMEOUT_TMEM_FULL, 8 + t)) return kFail;
+                tc_fence_after();
+                tmem_st_16x128b_x16(tO + kColP, pk);
+                FBB_TRACE(4 + u + 8 * t, g, 3);
+                tmem_wait_st();
+                tc_fence_before();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(p_ready(t));
+                FBB_TRACE(4 + u + 8 * t, g, 4);
+                lA += accA.x + accA.y;
+                lB += accB.x + accB.y;
+                return kDone;
+            };
+#pragma unroll 1
+            while (n > 0) {
+                // ---- the units that are all alike, then the ragged one
+                int got = kDone;
+#pragma unroll 1
+                for (; plain > 0; --plain, --n, ++g) {
+                    got = unit(std::false_type());
+                    if (got != kDone) break;
+                }
+                if (got == kDone && n > 0) {
+                    got = unit(std::true_type());
+                    if (got == kDone) {
+                        --n;
+                        ++g;
+                    }
+                }
+                ok = got != kFail;
                 if (!ok || n == 0) break;
-                // ---- the others, half a key block at a time from tensor memory: a block that exceeds a row's running maximum by
-                // more than 2^kLazyMax (raises them and rescales O and the sums) and the ragged last block (masks keys)
+                // ---- a block that exceeds a row's running maximum by more than 2^kLazyMax (raises them and rescales O and the sums),
+                // half of it at a time from tensor memory
                 const bool mask = plain == 0;
+                float2 accA = make_float2(0.f, 0.f), accB = make_float2(0.f, 0.f);
                 if (!mbar_wait(s_full(t), g & 1u, s_abort, DEV_TIMEOUT_TMEM_FULL, t)) { ok = false; break; }
                 tc_fence_after();
                 float mxA = -INFINITY, mxB = -INFINITY;
@@ -862,8 +931,6 @@ flash64_umma_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
                     tA = fmaxf(tA, mxA + lazy);
                     tB = fmaxf(tB, mxB + lazy);
                 }
-                accA = make_float2(0.f, 0.f);
-                accB = make_float2(0.f, 0.f);
 #pragma unroll 1
                 for (int h = 0; h < 2; ++h) {
                     uint32_t v[32], pk[16];

@@ -538,6 +538,26 @@ def test_flash_maxima_raised_block_after_block_into_a_strided_output(oracle, B, 
     status_ok()
 
 
+@pytest.mark.parametrize("raised", [False, True])
+@pytest.mark.parametrize("keys", [1, 63, 64, 65, 127, 128])
+@pytest.mark.parametrize("B,blocks,H", [(1, 1, 3), (2, 2, 5), (1, 4, 2), (3, 2, 64), (2, 4, 80)])
+def test_flash_last_key_block_of_every_width(oracle, B, blocks, H, keys, raised):
+    """A last key block with keys in its lower half only, in both halves, or full; as the only block, the second or the fourth; in
+    the one-tile and the two-tile kernel; with and without a maximum that this block has to raise."""
+    from fastbb_b200.attention import attention
+    N = 128 * (blocks - 1) + keys
+    g = torch.Generator().manual_seed(1000 * blocks + keys)
+    q, k, v = (torch.randn(B, N, H, 64, generator=g).half() for _ in range(3))
+    if raised:
+        q[:, ::3, :, 0] = 8.0
+        k[:, -1, :, 0] = 16.0  # 8 * 16 / 8 = 16 score units, 2^23, from the last key alone
+    out, check = padded((B, N, H, 64))
+    attention(q.to(dev()), k.to(dev()), v.to(dev()), out=out)
+    assert oracle.rel_l2(out.cpu().float(), oracle.attention(q, k, v)) < (2e-3 if raised else TOL_F32)
+    check()
+    status_ok()
+
+
 @pytest.mark.parametrize("B,N,H", [(37, 600, 4), (37, 513, 4), (20, 300, 16)])
 def test_flash_padding_warps_behind_a_working_item(oracle, B, N, H):
     """CTAs that take several tile groups, where a group with rows for all warps is followed by one that leaves some warps (or a
