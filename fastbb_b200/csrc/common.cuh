@@ -175,6 +175,11 @@ __device__ __forceinline__ void tma_store_4d(const void* map, uint32_t src, int 
 __device__ __forceinline__ void stmatrix_x4(uint32_t addr, uint32_t r0, uint32_t r1, uint32_t r2, uint32_t r3) {
     asm volatile("stmatrix.sync.aligned.m8n8.x4.shared.b16 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(r0), "r"(r1), "r"(r2), "r"(r3) : "memory");
 }
+__device__ __forceinline__ uint4 ld_shared_16(uint32_t addr) {
+    uint4 v;
+    asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(addr) : "memory");
+    return v;
+}
 // Announce `bytes` on the barrier (0: not at all) and load one box of each of two tensors, by one elected lane of a converged warp.
 __device__ __forceinline__ void tma_load_2d_two_warp(uint32_t bar, uint32_t bytes, uint32_t dst0, const void* map0, int x0, int y0, uint32_t dst1,
                                                      const void* map1, int x1, int y1) {
