@@ -163,6 +163,15 @@ def test_linear_matches_oracle(oracle, M, N, K, act, has_bias, has_res, variant)
     status_ok()
 
 
+def linear_form(M, N, K, epilogue=0, over_a=0):
+    """The form a linear() launch takes, spelled as in FBB_GEMM_FORCE."""
+    import ctypes
+    from fastbb_b200 import _lib
+    name = ctypes.create_string_buffer(16)
+    _lib.check(_lib.load().fbb_linear_form(M, N, K, epilogue, over_a, name, len(name)))
+    return name.value.decode()
+
+
 @pytest.mark.parametrize("form", ["s256", "s128", "p256", "p128", "w32", "w96", "w256", "w288", "w352", "w512"])
 def test_linear_every_tile_form_matches_oracle(oracle, form, monkeypatch):
     """The kernel has several forms (one CTA or a CTA pair per tile, 256- or 128-column tiles; wide pair items of 32 to
@@ -192,16 +201,17 @@ def test_linear_every_tile_form_matches_oracle(oracle, form, monkeypatch):
     status_ok()
 
 
-@pytest.mark.parametrize("bn", [32, 64, 128])
-@pytest.mark.parametrize("ctas", [1, 2, 4, 8])
+@pytest.mark.parametrize("ctas,bn", [(c, b) for c in (1, 2, 4, 8) for b in (32, 64, 128) if (c, b) != (1, 128)])
 def test_linear_split_form_matches_oracle(oracle, ctas, bn, monkeypatch):
     """The form whose tiles are shared by the CTAs of a cluster along K: row and column remainders, a ragged last k-block, shares
-    of unequal length, more k-blocks per CTA than the operand ring holds, one row, the residual updated in place."""
+    of unequal length, more k-blocks per CTA than the operand ring holds, one row, the residual updated in place. (One CTA on 128
+    columns is not a form: its threads would hold more of the epilogue than they have registers for.)"""
     from fastbb_b200.gemm import linear
     monkeypatch.setenv("FBB_GEMM_FORCE", f"k{ctas}x{bn}")
     g = torch.Generator().manual_seed(ctas * 1000 + bn)
     for M, N, K, act, variant, bias in [(257, 136, 520, None, "f32", True), (129, 200, 1096, "gelu", "f32", True), (1, 64, 512, None, "h", False),
-                                        (128, 8, 8 * 64 * ctas + 72, None, "f32", True), (383, 264, 1024, "gelu", "h", False)]:
+                                        (128, 8, 8 * 64 * ctas + 72, None, "f32", True), (128 if (ctas, bn) == (8, 32) else 383, 264, 1024, "gelu", "h", False)]:
+        assert linear_form(M, N, K, 1 if act == "gelu" else 0) == f"k{ctas}x{bn}"
         x = torch.randn(M, K, generator=g).half()
         w = (torch.randn(N, K, generator=g) / K ** 0.5).half()
         b = (0.1 * torch.randn(N, generator=g)).half() if bias else None
@@ -216,15 +226,6 @@ def test_linear_split_form_matches_oracle(oracle, ctas, bn, monkeypatch):
         assert oracle.rel_l2(y.cpu().float(), want) < (TOL_F16 if variant == "h" else TOL_F32), (M, N, K, act)
         check()
     status_ok()
-
-
-def linear_form(M, N, K, epilogue=0, over_a=0):
-    """The form a linear() launch takes, spelled as in FBB_GEMM_FORCE."""
-    import ctypes
-    from fastbb_b200 import _lib
-    name = ctypes.create_string_buffer(16)
-    _lib.check(_lib.load().fbb_linear_form(M, N, K, epilogue, over_a, name, len(name)))
-    return name.value.decode()
 
 
 @pytest.mark.parametrize("M", [1, 7, 8, 9, 33, 63, 64, 65, 120, 121, 127])
