@@ -1117,7 +1117,7 @@ static bool split_fits(const SplitClusters& most, int64_t M, int N, int K, int b
 // Time of the split form in us, fitted to measurements on B200 (back-to-back launches with dependent launch): a fixed part
 // per tile width and cluster size (start, the exchange of partials, output) and 0.19 us per k-block of the longest share.
 static double split_cost_us(int K, int bn, int s) {
-    static const double fixed[4][3] = {{2.1, 2.5, 4.0}, {2.7, 3.4, 4.8}, {3.1, 3.8, 6.4}, {3.9, 4.1, 6.4}};  // [log2 s][log2 bn / 32]
+    static const double fixed[4][3] = {{2.1, 2.5, 0.0 /* refused by split_fits */}, {2.7, 3.4, 4.8}, {3.1, 3.8, 6.4}, {3.9, 4.1, 6.4}};  // [log2 s][log2 bn / 32]
     const int num_kb = (K + BK - 1) / BK;
     return fixed[s == 8 ? 3 : s >> 1][bn >> 6] + 0.19 * (double)((num_kb + s - 1) / s);
 }
@@ -1567,13 +1567,13 @@ static LinearForm choose_form(int64_t M, int N, int K, bool swiglu, bool over_a)
     }
     // The split form: a candidate where its tiles times its cluster size fit the SMs at once, taken where its time (see
     // split_cost_us) is below that of the forms above, 2.7 us and 0.9 of the model's units of time. Measured on B200 (us,
-    // without / with): M = 257: N = 384, K = 1536 8.4 / 4.8 (two CTAs per tile of 32 columns), K = 384 5.2 / 3.2 (one);
-    // N = 1152, K = 384 4.4 / 3.2; N = 768, K = 3072 13.2 / 7.5; N = 1024, K = 4096 16.3 / 9.6; M = 1041: N = 768, K = 3072
-    // 14.3 / 10.2, K = 768 6.5 / 4.9; M = 2056, N = 384, K = 1536 10.3 / 7.5.
+    // without / with): M = 257: N = 384, K = 1536 8.4 / 5.0 (two CTAs per tile of 32 columns), K = 384 5.3 / 3.2 (one);
+    // N = 1152, K = 384 4.5 / 3.2; N = 768, K = 3072 13.2 / 7.5; N = 1024, K = 4096 16.3 / 9.7; M = 1041: N = 768, K = 3072
+    // 14.1 / 10.2, K = 768 6.5 / 4.9; M = 2056, N = 384, K = 1536 10.0 / 7.3.
     // Not where the output overlaps A: a row's columns are then several CTAs' tiles, and one may write what another has still to
     // read. (The persistent forms give up to 128 columns to one CTA, which has read its rows of A before it writes them.)
     int split_bn = 0, split_s = 0;
-    if (!swiglu && !over_a && ((M + BM - 1) / BM) * tn128 <= sms) {  // (its widest tiles, one CTA each, fit the SMs at once)
+    if (!swiglu && !over_a && ((M + BM - 1) / BM) * ((n_out + 63) / 64) <= sms) {  // (the fewest CTAs it takes: one on every 64 columns)
         const SplitClusters& most = split_max_clusters();
         const double unit_us = 0.37 * (double)((K + BK - 1) / BK) + 1.0;
         double split_best = 2.7 + 0.9 * unit_us * best;
