@@ -206,17 +206,6 @@ __device__ __forceinline__ void tma_load_2d_warp(uint32_t dst, const void* map, 
         ::"r"(dst), "l"(map), "r"(bar), "r"(x), "r"(y)
         : "memory");
 }
-__device__ __forceinline__ void tma_load_4d_expect_warp(uint32_t dst, const void* map, uint32_t bar, uint32_t bytes, int c0, int c1, int c2, int c3) {
-    asm volatile(
-        "{\n\t"
-        ".reg .pred q;\n\t"
-        "elect.sync _|q, 0xFFFFFFFF;\n\t"
-        "@q mbarrier.arrive.expect_tx.shared::cta.b64 _, [%2], %7;\n\t"
-        "@q cp.async.bulk.tensor.4d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5, %6}], [%2];\n\t"
-        "}\n"
-        ::"r"(dst), "l"(map), "r"(bar), "r"(c0), "r"(c1), "r"(c2), "r"(c3), "r"(bytes)
-        : "memory");
-}
 __device__ __forceinline__ void bulk_commit() { asm volatile("cp.async.bulk.commit_group;" ::: "memory"); }
 // Until the bulk stores committed by this thread have finished READING shared memory (the buffer may be rewritten).
 __device__ __forceinline__ void bulk_wait_read_all() { asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory"); }
@@ -262,11 +251,6 @@ __device__ __forceinline__ void tmem_ld_16x256b_x8(uint32_t taddr, uint32_t* r) 
     asm volatile("tcgen05.ld.sync.aligned.16x256b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];"
         : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]), "=r"(r[16]), "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]), "=r"(r[24]), "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
         : "r"(taddr)
-        : "memory");
-}
-__device__ __forceinline__ void tmem_st_16x256b_x8(uint32_t taddr, const uint32_t* r) {
-    asm volatile("tcgen05.st.sync.aligned.16x256b.x8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31, %32};"
-        ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]), "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15]), "r"(r[16]), "r"(r[17]), "r"(r[18]), "r"(r[19]), "r"(r[20]), "r"(r[21]), "r"(r[22]), "r"(r[23]), "r"(r[24]), "r"(r[25]), "r"(r[26]), "r"(r[27]), "r"(r[28]), "r"(r[29]), "r"(r[30]), "r"(r[31])
         : "memory");
 }
 // 16 columns at a time (8 registers): for the rare in-place rescale of O, which must not hold a whole tile in registers
@@ -357,11 +341,10 @@ __device__ __forceinline__ void umma_kblock_commit_warp(uint32_t d_tmem, uint64_
         : "memory");
 }
 // The same with commits to two barriers, accumulator overwritten (the Q K^T of one key block).
-__device__ __forceinline__ void umma_kblock_commit2_warp(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accumulate, uint32_t bar0,
-                                                         uint32_t bar1) {
+__device__ __forceinline__ void umma_kblock_commit2_warp(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t bar0, uint32_t bar1) {
     asm volatile(
         "{\n\t"
-        ".reg .pred p, q;\n\t"
+        ".reg .pred q;\n\t"
         ".reg .b64 a1, a2, a3, b1, b2, b3;\n\t"
         "add.s64 a1, %1, 2;\n\t"
         "add.s64 b1, %2, 2;\n\t"
@@ -369,16 +352,15 @@ __device__ __forceinline__ void umma_kblock_commit2_warp(uint32_t d_tmem, uint64
         "add.s64 b2, %2, 4;\n\t"
         "add.s64 a3, %1, 6;\n\t"
         "add.s64 b3, %2, 6;\n\t"
-        "setp.ne.b32 p, %4, 0;\n\t"
         "elect.sync _|q, 0xFFFFFFFF;\n\t"
-        "@q tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t"
+        "@q tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, 0;\n\t"
         "@q tcgen05.mma.cta_group::1.kind::f16 [%0], a1, b1, %3, 1;\n\t"
         "@q tcgen05.mma.cta_group::1.kind::f16 [%0], a2, b2, %3, 1;\n\t"
         "@q tcgen05.mma.cta_group::1.kind::f16 [%0], a3, b3, %3, 1;\n\t"
+        "@q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%4];\n\t"
         "@q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%5];\n\t"
-        "@q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%6];\n\t"
         "}\n"
-        ::"r"(d_tmem), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate), "r"(bar0), "r"(bar1)
+        ::"r"(d_tmem), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(bar0), "r"(bar1)
         : "memory");
 }
 // A from tensor memory (8 columns per K16 step), B MN-major (2048 bytes per step): eight steps and commits to two barriers.

@@ -518,7 +518,7 @@ flash64_umma_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
         auto issue_qk = [&](int it, int s, bool last) {
             const uint64_t qd = qd0 + (uint64_t)((it & 1) * (2 * kTileBytes >> 4));
             const uint64_t kd = kd0 + (uint64_t)(s * (kTileBytes >> 4));
-            umma_kblock_commit2_warp(dS, qd, kd, idesc_qk, 0u, s_full(t), k_empty(s));
+            umma_kblock_commit2_warp(dS, qd, kd, idesc_qk, s_full(t), k_empty(s));
             if (last) umma_commit_warp(q_empty(it & 1));  // this buffer may be loaded again
         };
         int it = 0, kb = 0, kb1 = 0;
