@@ -69,9 +69,11 @@ int launch_layernorm(const void* x, void* y, const void* w, const void* b, int64
 int launch_layernorm_split(const void* x, const void* w, const void* b, void* patches_out, void* cls_out, void* regs_out, int B, int N, int C,
                            int n_prefix, float eps, int apply_norm, int channel_major, cudaStream_t stream);
 
-// w_early: W (and nothing else) was written before the launch that precedes this one on the stream STARTED, so that its tiles may
-// be loaded ahead of the dependency wait. True inside a run of blocks: every kernel there starts its dependents only after its
-// own wait, so when a GEMM's CTAs start, everything before the launch in front of it is complete, and that launch writes no weights.
+// w_early: W (and nothing else) was complete before the launch that precedes this one on the stream STARTED, so that its tiles may
+// be loaded ahead of the dependency wait. True inside a run of blocks. A launch there writes no weights, so a GEMM's CTAs must
+// only not start before the stream's work ahead of the RUN is complete: the run's first launch (a LayerNorm) starts its dependents
+// after its own wait for that work, and no later launch can start before them. (Not more than that: the attention's side launch
+// starts its dependents before its own wait, so proj's CTAs may load W while the tiled attention launch still runs.)
 int launch_linear(const void* A, const void* W, void* C, const void* bias, const void* res, const void* gamma, int64_t M,
                   int N, int K, int64_t lda, int64_t ldw, int64_t ldc, int64_t ldr, int epilogue, int accumulate,
                   cudaStream_t stream, bool w_early = false);

@@ -398,6 +398,53 @@ def test_runner_descriptor_cache_follows_the_block(oracle):
     assert _lib_status() == (0, 0, 0, 0)
 
 
+@pytest.mark.parametrize("arch,tokens", [("vits14", 257), ("vits14", 5), ("vitb14", 1041), ("vitb14", 4097)])
+def test_weights_written_on_the_stream_right_before_a_run_of_blocks(oracle, arch, tokens):
+    """The GEMMs of a run of blocks may load weights ahead of their dependency wait. Weights that the stream writes directly before
+    the run, behind work that keeps it busy - by a copy, and by a launch of this library, which starts its dependents early -
+    must be the ones that the run uses. Sizes where the GEMMs share K among CTAs, and one with the attention's side launch."""
+    from fastbb_b200 import vit as V
+    from fastbb_b200.gemm import linear
+    _, fast = _fast_model(oracle, arch, "fh-g0")
+    blocks = fast.blocks[:2]
+    names = ("attn.qkv", "attn.proj", "mlp.fc1", "mlp.fc2")
+    weights = [b.get_submodule(n).weight for b in blocks for n in names]
+    old = [w.detach().clone() for w in weights]
+    g = torch.Generator("cuda").manual_seed(tokens)
+    C = weights[0].shape[1]
+    x = torch.randn(1, tokens, C, device="cuda:0", generator=g).half()
+    # new weights are products, so that linear() can write them: w = a . b^T
+    ab = [((0.02 * torch.randn(w.shape[0], 64, device="cuda:0", generator=g)).half(), torch.randn(w.shape[1], 64, device="cuda:0", generator=g).half() / 8)
+          for w in weights]
+    new = [linear(a, b) for a, b in ab]
+    busy = torch.randn(4096, 4096, device="cuda:0", generator=g).half()
+
+    def run():
+        y = x.clone()
+        assert V.run_stack(blocks, y, "fh", False)
+        return y
+
+    def put(values):
+        for w, v in zip(weights, values):
+            w.copy_(v)
+
+    with torch.no_grad():
+        before = run()
+        put(new)
+        torch.cuda.synchronize()
+        want = run()
+        assert not torch.equal(want, before)
+        for write in (lambda: put(new), lambda: [linear(a, b, out=w) for (a, b), w in zip(ab, weights)]):
+            for _ in range(5):
+                put(old)
+                torch.cuda.synchronize()
+                for _ in range(4):
+                    busy @ busy
+                write()
+                assert torch.equal(run(), want)
+    assert _lib_status() == (0, 0, 0, 0)
+
+
 def test_c_block_runner_direct_call_and_validation(oracle):
     """fbb_block_forward_f16 through ctypes on one block: equals run_block, updates x in place, rejects a scratch that is
     too small, a head count that does not match C, and a null weight."""
