@@ -228,6 +228,33 @@ def test_linear_split_form_matches_oracle(oracle, ctas, bn, monkeypatch):
     status_ok()
 
 
+@pytest.mark.parametrize("M,N,K", [(257, 384, 1536), (100, 1152, 384), (1041, 768, 768), (129, 72, 328)])
+def test_linear_split_form_with_row_strides(oracle, M, N, K):
+    """Every operand a part of wider rows, each with a stride of its own (the residual is another tensor than the output), and what
+    lies between the output's rows left alone."""
+    from fastbb_b200 import _lib
+    assert linear_form(M, N, K).startswith("k")
+    g = torch.Generator().manual_seed(M + N + K)
+
+    def rows(r, c, extra, off, fill=None):
+        buf = torch.randn(r, c + extra, generator=g).half().to(dev()) if fill is None else torch.full((r, c + extra), fill, dtype=torch.float16, device=dev())
+        return buf, buf[:, off:off + c]
+
+    _, x = rows(M, K, 24, 8)
+    wb, w = rows(N, K, 40, 16)
+    wb.div_(K ** 0.5)
+    _, res = rows(M, N, 8, 0)
+    buf, out = rows(M, N, 56, 32, CANARY)
+    b, gam = (0.1 * torch.randn(N, generator=g)).half(), (0.05 + 0.15 * torch.rand(N, generator=g)).half()
+    bd, gd = b.to(dev()), gam.to(dev())
+    _lib.check(_lib.load().fbb_linear_f16(x.data_ptr(), w.data_ptr(), out.data_ptr(), bd.data_ptr(), res.data_ptr(), gd.data_ptr(), M, N, K,
+                                          x.stride(0), w.stride(0), out.stride(0), res.stride(0), _lib.EPI_NONE, _lib.ACC_F32, _lib.stream_ptr(dev())))
+    assert oracle.rel_l2(out.cpu().float(), oracle.linear(x.cpu(), w.cpu(), b, res=res.cpu(), gamma=gam)) < TOL_F32
+    out.fill_(CANARY)
+    assert torch.all(buf == CANARY), "kernel wrote outside its output"
+    status_ok()
+
+
 @pytest.mark.parametrize("M", [1, 7, 8, 9, 33, 63, 64, 65, 120, 121, 127])
 def test_linear_split_form_of_fewer_rows_than_a_tile(oracle, M):
     """A tile of the split form loads no more rows of x than there are (to the next eight). What the rest of its shared memory
@@ -536,6 +563,23 @@ def test_flash_maxima_raised_block_after_block_into_a_strided_output(oracle, B, 
     assert oracle.rel_l2(out.cpu().float(), want) < 2e-3  # P and O are rounded to fp16 once each: 2 * 2^-11 at most, doubled
     out.fill_(CANARY)
     assert torch.all(buf == CANARY), "kernel wrote outside its output"
+    status_ok()
+
+
+@pytest.mark.parametrize("B,N,H", [(1, 257, 6), (2, 600, 5), (20, 300, 16), (1, 4097, 12)])
+def test_flash_output_of_other_dimension_orders(oracle, B, N, H):
+    """out= with its dimensions in [B, H, N, 64] and [N, B, H, 64] order in memory: the same bits as into a contiguous output."""
+    from fastbb_b200.attention import attention
+    g = torch.Generator().manual_seed(N + H)
+    q, k, v = (torch.randn(B, N, H, 64, generator=g).half().to(dev()) for _ in range(3))
+    want = attention(q, k, v)
+    rows = _sample_rows(N, seed=H)
+    assert oracle.rel_l2(want[:1, rows].cpu().float(), oracle.attention(q[:1, rows].cpu(), k[:1].cpu(), v[:1].cpu())) < TOL_F32
+    for shape, order in [((B, H, N, 64), (0, 2, 1, 3)), ((N, B, H, 64), (1, 0, 2, 3))]:
+        buf, check = padded(shape)
+        out = buf.permute(order)
+        assert attention(q, k, v, out=out) is out and torch.equal(out, want)
+        check()
     status_ok()
 
 
