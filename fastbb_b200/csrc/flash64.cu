@@ -23,20 +23,22 @@
 //                   has written P_t (fp16) back into tensor memory, O_t += P_t V_j (A from tensor memory, V as the
 //                   MN-major B operand, 8 x K16); O_t stays in tensor memory (fp32) over the key blocks of an item
 //   warps 4..11/12..19 softmax group t, 16 query rows per warp: tcgen05.ld 16x256b hands thread i the key pairs
-//                   8k + 2(i%4), +1 of rows i/4 and i/4 + 8 (the m16n8 accumulator fragment), so a row's maximum and sum
-//                   take two shuffles among the four threads that share it, and P (fp16 pairs) goes back with the
-//                   matching 16x128b store. The 128-key block is loaded at once; the maximum is taken with 3-input max,
-//                   p = 2^(s*scale*log2e - m) with packed f32x2 FMAs. The running maximum m is only raised when a block
-//                   exceeds it by more than 2^8 (then O_t and the running sum are rescaled in place, a rare event after
-//                   the first blocks); otherwise P is taken relative to the older maximum, which keeps it <= 256 and
-//                   exactly as accurate in fp16. The loop over an item's blocks holds only what every block needs: each
-//                   thread compares its own share of a row with the row's limit and the warp votes (no shuffles), and a
-//                   block that has to raise the maximum leaves for code that reads S again from tensor memory in halves; a
-//                   ragged last block has a masking copy of the loop's code behind it. An item's first block (which takes the maximum) stands before the loop, its
-//                   rows are written by 16-row TMA stores in the NEXT item's first block, behind that block's
-//                   exponentials, and Q has two buffers, so that neither tile stops between items. With one loop for all
-//                   of this and the write-out between items: 1531 / 213.6 / 81.8 us at N = 16385 / 6145 / 4097 (16 / 16 /
-//                   12 heads, back to back on one B200); now 1303 / 193.0 / 73.5.
+//                   8k + 2(i%4), +1 of rows i/4 and i/4 + 8 (the m16n8 accumulator fragment), and P (fp16 pairs) goes back
+//                   with the matching 16x128b store. The 128-key block is loaded at once; the maximum is taken with 3-input
+//                   max, p = 2^(s*scale*log2e - m) with packed f32x2 FMAs. The running maximum m is only raised when a block
+//                   exceeds it by more than 2^8 (then O_t and the running sum are rescaled in place, a rare event after the
+//                   first blocks); otherwise P is taken relative to the older maximum, which keeps it <= 256 and exactly as
+//                   accurate in fp16. The loop over an item's blocks holds only what every block needs: each thread compares
+//                   its own share of a row with the row's limit and the warp votes. What other blocks need stands outside it:
+//                   an item's first block (which takes the maximum, with two shuffles among the four threads that share a
+//                   row) before the loop; a ragged last block in a masking copy of the loop's code; a block that has to raise
+//                   the maximum in code that reads S again from tensor memory in halves. An item's rows are written by
+//                   16-row TMA stores in the NEXT item's first block, behind that block's exponentials, a CTA's last rows by
+//                   plain stores, and Q has two buffers, so that neither tile stops between items. One loop for all of this,
+//                   the write-out between items, one Q buffer / this form, us a call, in turn in one process, from CUDA graphs:
+//                   1496 / 1337 (1 x 16385 tokens x 16 heads), 217 / 198 (1 x 6145 x 16), 81.5 / 71.5 (1 x 4097 x 12),
+//                   13.8 / 11.5 (1 x 1041 x 12), 81.8 / 74.8 (4 x 1370 x 24), 59.0 / 52.5 (32 x 257 x 16), 6.9 / 6.2 (1 x 257 x
+//                   16).
 //                   Four softmax warps share each SM sub-partition and cover one another's waits (measured against
 //                   one-thread-per-row groups of four warps: 740 -> 849 TFLOP/s at N = 16385).
 // With NQ = 2 the two groups alternate on the tensor core (S of one tile is computed while the other tile is in its
@@ -49,17 +51,18 @@
 // variant is therefore at least as accurate as the reference's.
 // The kernel is bound by the exponentials, not the tensor core: 128 x 128 of them per S tile against 16 results per
 // clock per SM from the transcendental unit is twice the time of the tile's two matrix products (1024 vs 2 x 256 clocks).
-// Measured dynamics worth knowing before changing the pipeline: a softmax warp alone cannot saturate the transcendental
-// unit, so the two tiles run fastest half a period apart (2800 clocks per unit); in step, every phase collides with its
-// twin (3800 clocks). The half-period offset set at start-up is not stable: over some tens of units the later tile
-// catches up. CTAs that live for one group (<= ~130 units) mostly keep it; the persistent form loses part of what it
-// gains from the removed wave this way. Every way of forcing the offset that was built measured slower than letting the
-// tiles run free (N = 6145, 16 heads, 198-200 us free): strict turns around a whole unit (3100 clocks per unit); turns
-// around the exponential loop only, per SM sub-partition, so that one tile's load / maximum / store phases fall under the
-// other's exponentials (218 us: the two warps a tile has on a sub-partition do not saturate its transcendental unit on
-// their own, four contending warps use it better); a one-sided lock that only holds a tile back until the other is
-// 4/16 .. 14/16 of the way through its exponentials (201-212 us). Batching the exponentials in the source (arguments,
-// then exponentials, then sums) compiles to the same schedule; writing P back in two halves costs a second wait (212 us).
+// A launch of 6145 tokens x 16 heads keeps that unit 82 % busy over its active clocks, the tensor pipe 41 %. Measured dynamics
+// worth knowing before changing the pipeline: a softmax warp alone cannot saturate the unit, so the two tiles run fastest half a
+// period apart; in step, every phase collides with its twin. The half-period offset set at start-up is not stable: over some
+// tens of units the later tile catches up. CTAs that live for one group (<= ~130 units) mostly keep it; the persistent form
+// loses part of what it gains from the removed wave this way. On the older loop (clocks per unit 2800 half a period apart, 3800
+// in step; 198 - 200 us at 6145 tokens with 25 groups a head) every way of forcing the offset that was built measured slower than
+// letting the tiles run free: strict turns around a whole unit (3100 clocks per unit); turns around the exponential loop only,
+// per SM sub-partition (218 us: the two warps a tile has on a sub-partition do not saturate its unit on their own, four
+// contending warps use it better); a one-sided lock that only holds a tile back until the other is 4/16 .. 14/16 of the way
+// through its exponentials (201 - 212 us). So did writing P back in two halves (a second wait, 212 us).
+// Short launches (N <= 300, one tile per CTA) are chains of latencies: 1650 clocks from the dependency wait to the first Q and K in
+// shared memory, 650 more to S, 1200 - 1600 for a block's softmax, 1650 from the last P.V to the end.
 #include "common.cuh"
 #include <cstdlib>
 #include <type_traits>
@@ -74,14 +77,14 @@ constexpr int kKVStages = 4;
 constexpr int kTileBytes = 128 * 64 * 2;  // one [128 x 64] fp16 tile
 constexpr float kLazyMax = 8.0f;          // raise the running maximum only beyond 2^8
 // Key groups of eight whose exponentials a thread takes before the test of the running maximum is known: the test's vote then
-// costs no wait, and S_t is released that much later. Measured on B200 (us at N = 16385 / 6145 / 1041 tokens, 16 / 16 / 12
-// heads): 0 -> 1315 / 194.0 / 14.4, 2 -> 1332 / 194.3 / 13.9, 4 -> 1303 / 193.0 / 13.5, 8 -> 1324 / 190.4 / 13.7.
+// costs no wait, and S_t is released that much later. Measured on B200 (us at 1 x 16385 x 16 / 1 x 6145 x 16 / 1 x 1041 x 12 / 32 x
+// 257 x 16): 0 -> 1396 / 198 / 11.9 / 52.7, 2 -> 1360 / 195 / 11.6 / 52.5, 4 -> 1337 / 198 / 11.5 / 52.5, 8 -> 1386 / 200 / 11.8 / 53.4.
 constexpr int kEarly = 4;
 // Register split of the 640-thread (NQ = 2) kernel. It is launched with 96 registers per thread (the most 20 warps can
 // get); setmaxnreg.inc WAITS until the CTA's own pool has the registers, so the split must fit in that pool or the
 // kernel never starts its softmax: 128 * kRegsCtl + 512 * kRegsSoftmax <= 640 * 96. A softmax thread holds 64 scores and up to
-// 32 packed probabilities; 104 hold them without spilling, and the issuers keep their loop state in registers with 56
-// (us at N = 16385 / 6145 / 4097, 16 / 16 / 12 heads: 1303 / 193 / 73.5; with 32 / 112: 1358 / 200 / 76.5).
+// 32 packed probabilities; 104 hold them (one predicate word spills), and the issuers keep their loop state in registers with 56 (us at
+// 1 x 16385 x 16 / 1 x 6145 x 16 / 4 x 1370 x 24: 1337 / 198 / 74.8; with 32 / 112: 1368 / 202 / 80.1).
 constexpr int kRegsCtl = 56, kRegsSoftmax = 104;
 static_assert(128 * kRegsCtl + 512 * kRegsSoftmax <= 640 * 96, "setmaxnreg split exceeds the CTA's register pool");
 

@@ -1567,7 +1567,7 @@ static LinearForm choose_form(int64_t M, int N, int K, bool swiglu, bool over_a)
     }
     // The split form: a candidate where its tiles times its cluster size fit the SMs at once, taken where its time (see
     // split_cost_us) is below that of the forms above, 2.7 us and 0.9 of the model's units of time. Measured on B200 (us,
-    // without / with): M = 257: N = 384, K = 1536 8.4 / 5.0 (two CTAs per tile of 32 columns), K = 384 5.3 / 3.2 (one);
+    // without / with): M = 257: N = 384, K = 1536 8.4 / 5.0 (four CTAs per tile of 64 columns), K = 384 5.3 / 3.2 (one on 32);
     // N = 1152, K = 384 4.5 / 3.2; N = 768, K = 3072 13.2 / 7.5; N = 1024, K = 4096 16.3 / 9.7; M = 1041: N = 768, K = 3072
     // 14.1 / 10.2, K = 768 6.5 / 4.9; M = 2056, N = 384, K = 1536 10.0 / 7.3.
     // Not where the output overlaps A: a row's columns are then several CTAs' tiles, and one may write what another has still to
